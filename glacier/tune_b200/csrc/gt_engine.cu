@@ -1,6 +1,6 @@
 // C ABI of libglaciertune_b200.so (declared in include/glaciertune_b200.h): engine, weight upload,
 // adapters, projection forward / backward.  Host-side orchestration only; kernels are in
-// gt_fp32_kernels.cu (CUDA cores) and gt_umma_gemm.cu (tcgen05).
+// gt_fp32_kernels.cu, gt_exact_gemm.cu (fp32 accuracy) and gt_umma_gemm.cu (tcgen05).
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -388,16 +388,33 @@ int forward_device(gt_engine *e, const gt_weight *w, gt_adapter *ad, const float
     if (paired_path(e, w)) {
         int prc = paired_forward_base(e, w, Xd, Yd, T);
         if (prc != GT_OK) return prc;
-    } else {
-        GT_LAUNCH(e, launch_gemm_fp32_fwd(wd.qtype, wd.data, Xd, Yd, nullptr, wd.bias, T, N, K, e->stream));
     }
     if (use_lora) {
         int rc = compute_low(e, &ad, 1, Xd, nullptr, 0, T, K);
         if (rc != GT_OK) return rc;
-        GT_LAUNCH(e, launch_lora_delta_fp32(low_of(ad), ad->B, Yd, nullptr, T, N, ad->rank, ad->scaling, ad->b_nonzero, e->stream));
-    } else if (ad) {
-        ad->low_T = 0;
     }
+    if (!paired_path(e, w)) {
+        ExactGemm g;
+        g.qtype = wd.qtype;
+        g.w = wd.data;
+        g.act = Xd;
+        g.out = Yd;
+        g.bias = wd.bias;
+        g.T = T;
+        g.N = N;
+        g.K = K;
+        if (use_lora) {
+            g.lora_act = low_of(ad);
+            g.lora_w = ad->B;
+            g.scale = ad->scaling;
+            g.R = ad->rank;
+            g.flag = ad->b_nonzero;
+        }
+        GT_LAUNCH(e, launch_exact_gemm(g, e->sm_count, e->stream));
+    } else if (use_lora) {
+        GT_LAUNCH(e, launch_lora_delta_fp32(low_of(ad), ad->B, Yd, nullptr, T, N, ad->rank, ad->scaling, ad->b_nonzero, e->stream));
+    }
+    if (!use_lora && ad) ad->low_T = 0;
     return GT_OK;
 }
 
@@ -608,8 +625,6 @@ int backward_device(gt_engine *e, const gt_weight *w, gt_adapter *ad, const floa
     if (paired) {      // the base product writes (or adds into) dX itself
         int prc = paired_backward_base(e, w, dYd, dXd, T, assign);
         if (prc != GT_OK) return prc;
-    } else if (assign && dXd) {
-        GT_LAUNCH(e, launch_fill_rows(dXd, nullptr, T, K, e->stream));
     }
     if (use_lora) {
         const bool lora = true;
@@ -617,9 +632,27 @@ int backward_device(gt_engine *e, const gt_weight *w, gt_adapter *ad, const floa
         const int ld16 = round8(N);
         int rc = lora_backward_group(e, 1, &w, &ad, &lora, &dYd, Xd, &no16, &ld16, T, reuse_low, nullptr);
         if (rc != GT_OK) return rc;
-        if (dXd) GT_LAUNCH(e, launch_lora_dx_fp32(dlow_of(ad, T), ad->A, dXd, ad->scaling, T, K, ad->rank, e->stream));
+        if (paired) GT_LAUNCH(e, launch_lora_dx_fp32(dlow_of(ad, T), ad->A, dXd, ad->scaling, T, K, ad->rank, e->stream));
     }
-    if (dXd && !paired) GT_LAUNCH(e, launch_gemm_fp32_bwd(wd.qtype, wd.data, dYd, dXd, T, N, K, e->stream));
+    if (dXd && !paired) {
+        ExactGemm g;
+        g.qtype = wd.qtype;
+        g.w = wd.data;
+        g.backward = 1;
+        g.act = dYd;
+        g.out = dXd;
+        g.assign = assign ? 1 : 0;
+        g.T = T;
+        g.N = N;
+        g.K = K;
+        if (use_lora) {
+            g.lora_act = dlow_of(ad, T);
+            g.lora_w = ad->A;
+            g.scale = ad->scaling;
+            g.R = ad->rank;
+        }
+        GT_LAUNCH(e, launch_exact_gemm(g, e->sm_count, e->stream));
+    }
     return GT_OK;
 }
 
@@ -1513,7 +1546,17 @@ int gt_launch_gemm_batch(gt_engine *e, const gt_weight *w, float *dY_out, const 
     GT_CUDA(cudaSetDevice(e->device));
     const int N = w->dev.N, K = w->dev.K;
     if (!tensor_path(e, w)) {
-        GT_CUDA(launch_gemm_fp32_fwd(w->dev.qtype, w->dev.data, dX_in, dY_out, d_residual, w->dev.bias, batch, N, K, e->stream));
+        ExactGemm g;
+        g.qtype = w->dev.qtype;
+        g.w = w->dev.data;
+        g.act = dX_in;
+        g.out = dY_out;
+        g.residual = d_residual;
+        g.bias = w->dev.bias;
+        g.T = batch;
+        g.N = N;
+        g.K = K;
+        GT_CUDA(launch_exact_gemm(g, e->sm_count, e->stream));
         return GT_OK;
     }
     float *yd = dY_out;

@@ -1,5 +1,5 @@
-// CUDA-core kernels: exact dequantization, the fp32 validation GEMMs, and the rank-r LoRA products
-// (low = X*A, dB, dLow, dA) with fp32 accumulation.  The tensor-core GEMMs live in gt_umma_gemm.cu.
+// CUDA-core kernels: exact dequantization and the rank-r LoRA products (low = X*A, dB, dLow, dA) with fp32
+// accumulation.  The GEMMs live in gt_umma_gemm.cu (16-bit operands) and gt_exact_gemm.cu (fp32 accuracy).
 #include "gt_internal.h"
 #include "gt_ptx.cuh"
 #include "gt_quant.cuh"
@@ -53,141 +53,6 @@ cudaError_t launch_dequant_rows(int qt, const uint8_t *w, int K, int64_t row0, i
     else if (qt == kTypeQ40) k_dequant_rows<kTypeQ40><<<blocks, threads, 0, s>>>(w, K, row0, nrows, out);
     else if (qt == kTypeQ80) k_dequant_rows<kTypeQ80><<<blocks, threads, 0, s>>>(w, K, row0, nrows, out);
     else k_dequant_rows<kTypeF32><<<blocks, threads, 0, s>>>(w, K, row0, nrows, out);
-    return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------------------------------------
-// fp32 validation GEMMs (CUDA cores, exact weights).  64x64 output tile, 16-deep slabs, 4x4 per thread.
-// Weights are addressed as a flat element stream so tensors whose rows are not whole super-blocks work too.
-// ------------------------------------------------------------------------------------------------
-constexpr int FT = 64, FS = 16;
-
-template <int QT>
-__global__ void __launch_bounds__(256) k_gemm_fp32_fwd(const uint8_t *__restrict__ w, const float *__restrict__ X,
-                                                       float *__restrict__ Y, float *__restrict__ residual,
-                                                       const float *__restrict__ bias, int T, int N, int K) {
-    __shared__ float Xs[FS][FT + 4];
-    __shared__ float Ws[FS][FT + 4];
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int n0 = blockIdx.x * FT, t0 = blockIdx.y * FT;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += FS) {
-        {   // X tile: 64 tokens x 16 k; thread -> token tid/4, 4 consecutive k
-            const int t = t0 + (tid >> 2), kk = (tid & 3) * 4;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int k = k0 + kk + j;
-                Xs[kk + j][tid >> 2] = (t < T && k < K) ? X[(int64_t)t * K + k] : 0.f;
-            }
-            const int n = n0 + (tid >> 2);
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int k = k0 + kk + j;
-                Ws[kk + j][tid >> 2] = (n < N && k < K) ? decode_flat<QT>(w, (int64_t)n * K + k) : 0.f;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < FS; k++) {
-            float xv[4], wv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) xv[i] = Xs[k][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) wv[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xv[i], wv[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int t = t0 + ty * 4 + i;
-        if (t >= T) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n >= N) continue;
-            float v = acc[i][j];
-            if (bias) v += bias[n];
-            if (residual) residual[(int64_t)t * N + n] += v;
-            if (Y) Y[(int64_t)t * N + n] = v;
-        }
-    }
-}
-
-template <int QT>
-__global__ void __launch_bounds__(256) k_gemm_fp32_bwd(const uint8_t *__restrict__ w, const float *__restrict__ dY,
-                                                       float *__restrict__ dX, int T, int N, int K) {
-    __shared__ float Gs[FS][FT + 4];   // dY tile  [n][token]
-    __shared__ float Ws[FS][FT + 4];   // W tile   [n][k]
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int k0 = blockIdx.x * FT, t0 = blockIdx.y * FT;
-    float acc[4][4] = {};
-    for (int n0 = 0; n0 < N; n0 += FS) {
-        {
-            const int t = t0 + (tid >> 2), nn = (tid & 3) * 4;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int n = n0 + nn + j;
-                Gs[nn + j][tid >> 2] = (t < T && n < N) ? dY[(int64_t)t * N + n] : 0.f;
-            }
-            const int n = n0 + (tid >> 4), kk = (tid & 15) * 4;
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const int k = k0 + kk + j;
-                Ws[tid >> 4][kk + j] = (n < N && k < K) ? decode_flat<QT>(w, (int64_t)n * K + k) : 0.f;
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int n = 0; n < FS; n++) {
-            float gv[4], wv[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) gv[i] = Gs[n][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) wv[j] = Ws[n][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(gv[i], wv[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int t = t0 + ty * 4 + i;
-        if (t >= T) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int k = k0 + tx * 4 + j;
-            if (k < K) dX[(int64_t)t * K + k] += acc[i][j];
-        }
-    }
-}
-
-cudaError_t launch_gemm_fp32_fwd(int qt, const uint8_t *w, const float *X, float *Y, float *residual, const float *bias,
-                                 int T, int N, int K, cudaStream_t s) {
-    if (T <= 0 || N <= 0) return cudaSuccess;
-    dim3 grid((N + FT - 1) / FT, (T + FT - 1) / FT);
-    if (qt == kTypeQ4K) k_gemm_fp32_fwd<kTypeQ4K><<<grid, 256, 0, s>>>(w, X, Y, residual, bias, T, N, K);
-    else if (qt == kTypeQ6K) k_gemm_fp32_fwd<kTypeQ6K><<<grid, 256, 0, s>>>(w, X, Y, residual, bias, T, N, K);
-    else if (qt == kTypeF16) k_gemm_fp32_fwd<kTypeF16><<<grid, 256, 0, s>>>(w, X, Y, residual, bias, T, N, K);
-    else if (qt == kTypeQ40) k_gemm_fp32_fwd<kTypeQ40><<<grid, 256, 0, s>>>(w, X, Y, residual, bias, T, N, K);
-    else if (qt == kTypeQ80) k_gemm_fp32_fwd<kTypeQ80><<<grid, 256, 0, s>>>(w, X, Y, residual, bias, T, N, K);
-    else k_gemm_fp32_fwd<kTypeF32><<<grid, 256, 0, s>>>(w, X, Y, residual, bias, T, N, K);
-    return cudaGetLastError();
-}
-cudaError_t launch_gemm_fp32_bwd(int qt, const uint8_t *w, const float *dY, float *dX, int T, int N, int K, cudaStream_t s) {
-    if (T <= 0 || K <= 0) return cudaSuccess;
-    dim3 grid((K + FT - 1) / FT, (T + FT - 1) / FT);
-    if (qt == kTypeQ4K) k_gemm_fp32_bwd<kTypeQ4K><<<grid, 256, 0, s>>>(w, dY, dX, T, N, K);
-    else if (qt == kTypeQ6K) k_gemm_fp32_bwd<kTypeQ6K><<<grid, 256, 0, s>>>(w, dY, dX, T, N, K);
-    else if (qt == kTypeF16) k_gemm_fp32_bwd<kTypeF16><<<grid, 256, 0, s>>>(w, dY, dX, T, N, K);
-    else if (qt == kTypeQ40) k_gemm_fp32_bwd<kTypeQ40><<<grid, 256, 0, s>>>(w, dY, dX, T, N, K);
-    else if (qt == kTypeQ80) k_gemm_fp32_bwd<kTypeQ80><<<grid, 256, 0, s>>>(w, dY, dX, T, N, K);
-    else k_gemm_fp32_bwd<kTypeF32><<<grid, 256, 0, s>>>(w, dY, dX, T, N, K);
     return cudaGetLastError();
 }
 

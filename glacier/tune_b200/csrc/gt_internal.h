@@ -46,9 +46,24 @@ struct WeightDev {
 // ---- CUDA-core kernels (gt_fp32_kernels.cu) -------------------------------------------------------------
 cudaError_t launch_q6k_repack(const uint8_t *gguf_blocks, uint8_t *dev_blocks, int64_t nblocks, cudaStream_t s);
 cudaError_t launch_dequant_rows(int qt, const uint8_t *w, int K, int64_t row0, int64_t nrows, float *out, cudaStream_t s);
-cudaError_t launch_gemm_fp32_fwd(int qt, const uint8_t *w, const float *X, float *Y, float *residual, const float *bias,
-                                 int T, int N, int K, cudaStream_t s);
-cudaError_t launch_gemm_fp32_bwd(int qt, const uint8_t *w, const float *dY, float *dX, int T, int N, int K, cudaStream_t s);
+// ---- fp32-accurate GEMMs on exact weights, any type and shape (gt_exact_gemm.cu)
+struct ExactGemm {
+    int qtype = 0;
+    const uint8_t *w = nullptr;
+    int backward = 0;                 // 0: out = act W^T + bias + lora (and residual += it); 1: out (+)= act W + lora
+    const float *act = nullptr;       // X [T, K] / dY [T, N]
+    float *out = nullptr;             // forward: may be null when residual is given
+    float *residual = nullptr;        // forward only
+    const float *bias = nullptr;      // forward only
+    int assign = 0;                   // backward: out is written, not added to
+    int T = 0, N = 0, K = 0;
+    // rank-r term (optional): scale * lora_act [T, R] * (forward: lora_w = B [R, N]; backward: lora_w^T, A [K, R])
+    const float *lora_act = nullptr, *lora_w = nullptr;
+    float scale = 0.f;
+    int R = 0;
+    const int *flag = nullptr;        // device int: 0 leaves the rank-r term out
+};
+cudaError_t launch_exact_gemm(const ExactGemm &g, int sm_count, cudaStream_t s);
 
 // LoRA (all fp32 arithmetic).  A is [K, R] row-major, B is [R, N] row-major.  Kernels handle ranks
 // [r0, r0+16) of R per launch.
