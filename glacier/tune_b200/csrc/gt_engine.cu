@@ -176,6 +176,71 @@ bool group_tensor_ok(const gt_engine *e, int n, const gt_weight *const *w) {
     return true;
 }
 
+// Few tokens (bf16 mode): the projections are bound by streaming the packed weights, which the warp-level kernel does
+// several times faster than the CTA-wide tensor-core kernels.
+bool decode_ok(const gt_engine *e, int n, bool dual, const gt_weight *const *w, const float *Xd, int T) {
+    if (e->math_mode != GT_MATH_BF16 || (reinterpret_cast<uintptr_t>(Xd) & 15) != 0 || n > kMaxGroup) return false;
+    const WeightDev *wd[kMaxGroup];
+    for (int j = 0; j < n; j++) wd[j] = &w[j]->dev;
+    return decode_group_ok(wd, n, dual, T, e->sm_count);
+}
+
+// One launch for the group (plus one for the adapters' X*A).  hidden != nullptr: gate | up, hidden = SiLU(Y_0) * Y_1, and
+// either Y_j may be null.
+int decode_forward(gt_engine *e, int n, const gt_weight *const *w, gt_adapter *const *ad, const bool *lora, const float *Xd, float *const *Yd,
+                   float *hidden, int T) {
+    const int K = w[0]->dev.K;
+    gt_adapter *with[kMaxGroup];
+    int n_with = 0;
+    bool few = true;
+    for (int j = 0; j < n; j++) {
+        if (!lora[j]) continue;
+        with[n_with++] = ad[j];
+        few = few && low_few_ok(T, ad[j]->rank);
+    }
+    if (n_with && few) {
+        LoraXaJob jobs[kMaxGroup];
+        GT_CUDA(e->low_parts.reserve(kMaxGroup * low_few_floats(8, 64) * sizeof(float)));
+        for (int j = 0; j < n_with; j++) {
+            gt_adapter *a = with[j];
+            GT_CUDA(a->low.reserve(2 * low_bytes(a, T)));
+            a->low_T = T;
+            a->dlow_clean = false;
+            jobs[j] = LoraXaJob{a->A, (float *)e->low_parts.p + j * low_few_floats(8, 64), a->rank};
+        }
+        GT_LAUNCH(e, launch_low_few(Xd, jobs, n_with, T, K, e->stream));
+    } else if (n_with) {
+        int rc = compute_low(e, with, n_with, Xd, nullptr, 0, T, K);
+        if (rc != GT_OK) return rc;
+    }
+    DecodeMember m[kMaxGroup];
+    for (int j = 0, k = 0; j < n; j++) {
+        m[j].w = &w[j]->dev;
+        m[j].out = Yd[j];
+        if (lora[j]) {
+            m[j].low = few ? (const float *)e->low_parts.p + k++ * low_few_floats(8, 64) : low_of(ad[j]);
+            m[j].low_out = few ? low_of(ad[j]) : nullptr;
+            m[j].B = ad[j]->B;
+            m[j].scale = ad[j]->scaling;
+            m[j].R = ad[j]->rank;
+            m[j].flag = ad[j]->b_nonzero;
+        }
+        e->gemm_flops += 2.0 * (double)T * (double)w[j]->dev.N * (double)K;
+    }
+    cudaEvent_t ea = nullptr, eb = nullptr;
+    if (e->profile) {
+        ea = next_event(e);
+        eb = next_event(e);
+        if (ea) cudaEventRecord(ea, e->stream);
+    }
+    cudaError_t ce = launch_decode(m, n, Xd, T, n_with > 0 && few && !e->profile, hidden != nullptr, hidden, e->sm_count, e->status, e->stream);
+    if (e->profile && eb) cudaEventRecord(eb, e->stream);
+    e->gemm_launches += 1;
+    e->kernel_launches += 1;
+    if (ce != cudaSuccess) return fail(GT_ERR_CUDA, "few-token forward launch failed: %s", cudaGetErrorString(ce));
+    return GT_OK;
+}
+
 // Y_j = X * W_j^T (+ bias_j) (+ lora_j) for 1..3 projections that read the same X.  Tensor-core path: one pass over X
 // (16-bit copy + every adapter's X*A), one GEMM launch.  Anything else runs member by member.
 // x16_ready (bf16 mode, members on the tensor path): the input already exists as bf16 [T, K] - nothing is cast, the
@@ -201,40 +266,7 @@ int forward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adap
     }
     const int K = w[0]->dev.K;
     const int fp16 = e->math_mode == GT_MATH_FP16;
-    // Few tokens: the projection is bound by streaming the packed weights, which the warp-level kernel does several
-    // times faster than the CTA-wide tensor-core kernel; the adapter term is added by the exact rank-r kernel.
-    bool stream = !x16_ready && e->math_mode == GT_MATH_BF16 && (reinterpret_cast<uintptr_t>(Xd) & 15) == 0;
-    for (int j = 0; j < n && stream; j++) stream = stream_fwd_ok(&w[j]->dev, T);
-    if (stream) {
-        gt_adapter *with[kMaxGroup];
-        int n_with = 0;
-        for (int j = 0; j < n; j++)
-            if (lora[j]) with[n_with++] = ad[j];
-        if (n_with) {
-            int rc = compute_low(e, with, n_with, Xd, nullptr, 0, T, K);
-            if (rc != GT_OK) return rc;
-        }
-        for (int j = 0; j < n; j++) {
-            const WeightDev &wd = w[j]->dev;
-            GT_LAUNCH(e, launch_fill_rows(Yd[j], wd.bias, T, wd.N, e->stream));      // the kernel adds into Y
-            cudaEvent_t ea = nullptr, eb = nullptr;
-            if (e->profile) {
-                ea = next_event(e);
-                eb = next_event(e);
-                if (ea) cudaEventRecord(ea, e->stream);
-            }
-            cudaError_t ce = launch_stream_fwd(&wd, Xd, Yd[j], T, e->sm_count, e->status, e->trace, e->stream);
-            if (e->profile && eb) cudaEventRecord(eb, e->stream);
-            e->gemm_launches += 1;
-            e->kernel_launches += 1;
-            e->gemm_flops += 2.0 * (double)T * (double)wd.N * (double)K;
-            if (ce != cudaSuccess) return fail(GT_ERR_CUDA, "streaming forward launch failed: %s", cudaGetErrorString(ce));
-            if (lora[j])
-                GT_LAUNCH(e, launch_lora_delta_fp32(low_of(ad[j]), ad[j]->B, Yd[j], nullptr, T, wd.N, ad[j]->rank, ad[j]->scaling,
-                                                    ad[j]->b_nonzero, e->stream));
-        }
-        return GT_OK;
-    }
+    if (!x16_ready && decode_ok(e, n, false, w, Xd, T)) return decode_forward(e, n, w, ad, lora, Xd, Yd, nullptr, T);
     if (!x16_ready) GT_CUDA(e->x16.reserve((size_t)T * K * 2));
     const void *act16 = x16_ready ? x16_ready : e->x16.p;
     UmmaLaunch m[kMaxGroup];
@@ -707,6 +739,24 @@ int ffn_forward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *cons
         float *yd = Yd;
         return forward_group_device(e, 1, w + 2, ad ? ad + 2 : nullptr, nullptr, &yd, T, flags, hidden16);
     }
+    if (Yd && !hidden16 && w[0]->dev.N == w[1]->dev.N && decode_ok(e, 2, true, w, Xd, T)) {
+        // few tokens: gate | up and the product in one launch, gate and up written only where the caller wants them
+        float *h = hidden_d;
+        if (!h) {
+            GT_CUDA(e->ffn[2].reserve(bf));
+            h = (float *)e->ffn[2].p;
+        }
+        bool lora[2];
+        for (int j = 0; j < 2; j++) {
+            lora[j] = ad && ad[j] && !(flags & GT_FLAG_NO_LORA) && ad[j]->rank > 0 && ad[j]->scaling != 0.f;
+            if (ad && ad[j] && !lora[j]) ad[j]->low_T = 0;
+            if (ad && ad[j]) ad[j]->xkeep_T = 0;
+        }
+        float *gu[2] = {gate_d, up_d};
+        int rc = decode_forward(e, 2, w, ad, lora, Xd, gu, h, T);
+        if (rc != GT_OK) return rc;
+        return forward_group_device(e, 1, w + 2, ad ? ad + 2 : nullptr, h, &Yd, T, flags);
+    }
     float *bufs[3] = {gate_d, up_d, hidden_d};
     for (int i = 0; i < 3; i++) {
         if (!bufs[i] && !(i == 2 && fold)) {      // folded: the fp32 product is written only where the caller wants it
@@ -978,6 +1028,7 @@ int gt_engine_create(const gt_config *cfg, gt_engine **out) {
     if (ce == cudaSuccess && cfg && cfg->max_tokens > 0 && cfg->max_features > 0) {
         const size_t T = (size_t)cfg->max_tokens, F = (size_t)cfg->max_features;
         ce = e->x16.reserve(T * F * 2);
+        if (ce == cudaSuccess) ce = e->low_parts.reserve(kMaxGroup * low_few_floats(8, 64) * sizeof(float));
         if (ce == cudaSuccess) ce = e->dy16.reserve(T * (F + 64) * 2 + 3 * 256);
         for (int i = 0; i < 3 && ce == cudaSuccess; i++) ce = e->ffn[i].reserve(T * F * sizeof(float));
         if (ce == cudaSuccess) logf(GT_LOG_INFO, "engine on device %d: scratch reserved for %zu tokens x %zu features (%.1f MB)", dev, T, F,
@@ -998,7 +1049,7 @@ int gt_engine_destroy(gt_engine *e) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     if (e->s_h2d) cudaStreamSynchronize(e->s_h2d);
     if (e->s_d2h) cudaStreamSynchronize(e->s_d2h);
-    Scratch *all[] = {&e->x16, &e->dy16, &e->dlow, &e->ytmp, &e->pair_tmp, &e->ffn[0], &e->ffn[1], &e->ffn[2], &e->ce, &e->ce_host, &e->attn};
+    Scratch *all[] = {&e->x16, &e->dy16, &e->dlow, &e->ytmp, &e->pair_tmp, &e->ffn[0], &e->ffn[1], &e->ffn[2], &e->ce, &e->ce_host, &e->attn, &e->low_parts};
     for (Scratch *s : all) s->release();
     for (HostSlot &sl : e->slots) {
         for (Scratch &b : sl.in) b.release();

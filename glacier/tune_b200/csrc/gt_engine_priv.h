@@ -89,6 +89,7 @@ struct gt_engine {
     Scratch x16, dy16, dlow, ytmp, pair_tmp;
     Scratch ce, ce_host;         // LM-head cross-entropy: logits / probability tiles and per-token state; host staging
     Scratch attn;                // attention: log-sum-exp rows and the dO.O row sums
+    Scratch low_parts;           // partial sums of X*A of the few-token forward
     Scratch ffn[3];              // gate, up, hidden (forward) / dHidden, dGate, dUp (backward) of the fused FFN calls
     // Host-buffer calls: a ring of staging slots and two copy streams, so that the upload of one call, the kernels
     // of the previous one and the download of the one before run at the same time (GT_FLAG_HOST_ASYNC), and a

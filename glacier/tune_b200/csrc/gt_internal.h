@@ -39,7 +39,7 @@ struct WeightDev {
     bool tma_ok = false;          // row-aligned and tensor maps built
     CUtensorMap tm_hdr, tm_q0, tm_q1;   // 2-D byte maps over [N, row_bytes], boxes of 64 rows (backward raw stages)
     CUtensorMap tm_hdr_f, tm_q0_f, tm_q1_f;   // the same with boxes of 128 rows (forward raw stages: half as many copies)
-    CUtensorMap tm_rows;                // Q4_K: 32-bit words over [N, row_bytes / 4], boxes of 16 rows x 288 bytes (two blocks)
+    CUtensorMap tm_rows;                // 32-bit words over [N, row_bytes / 4], boxes of 16 rows x two Q4_K blocks / one Q6_K block
     CUtensorMap tm_blk_f, tm_blk_b;     // whole super-blocks: boxes of one block x 256 rows / x 64 rows (few-token kernel)
 };
 
@@ -200,12 +200,26 @@ struct EngineView {
     int *status;       // device int[4], bounded-wait codes of the tensor-core kernels
     void *mutex;       // std::mutex * serialising calls on the engine
 };
-// ---- weight-streaming forward projection for few tokens (gt_stream_gemm.cu): warp-level MMAs on the quantized
-// integers, scales applied per sub-block on the partial sums.  Q4_K, whole 256-wide rows, T <= stream_max_tokens().
+// ---- weight-streaming forward projections for few tokens (gt_decode.cu): up to three members that share X in one launch,
+// bias, rank-r term and (dual: members 0 and 1) SiLU(out_0) * out_1 included.  T <= stream_max_tokens().
+struct DecodeMember {
+    const WeightDev *w = nullptr;
+    float *out = nullptr;                    // [T, N]; may be null in a dual launch
+    const float *low = nullptr, *B = nullptr;      // rank-r term: scale * low [T, R] B [R, N]
+    float *low_out = nullptr;                // given: low holds launch_low_few's partial sums, and their sum is kept here
+    float scale = 0.f;
+    int R = 0;
+    const int *flag = nullptr;               // device int: 0 leaves the rank-r term out
+};
 int stream_max_tokens();
-bool stream_fwd_ok(const WeightDev *w, int T);
-cudaError_t launch_stream_fwd(const WeightDev *w, const float *X, float *Y_prefilled, int T, int sm_count, int *status, void *trace,
-                              cudaStream_t s);
+bool decode_group_ok(const WeightDev *const *w, int n, bool dual, int T, int sm_count);
+// x_early: the kernel launched right before is launch_low_few on the same X (then X is complete when this one starts)
+cudaError_t launch_decode(const DecodeMember *m, int n, const float *X, int T, bool x_early, bool dual, float *hidden, int sm_count, int *status,
+                          cudaStream_t s);
+// X A for up to three adapters as partial sums of low_few_floats() values each, written (not added), exact fp32
+size_t low_few_floats(int T, int R);
+bool low_few_ok(int T, int R);
+cudaError_t launch_low_few(const float *X, const LoraXaJob *jobs, int n, int T, int K, cudaStream_t s);
 
 // ---- layer glue launchers used inside the library (gt_glue.cu)
 cudaError_t launch_swiglu_fwd(const float *gate, const float *up, float *hidden, int64_t n, int sm_count, cudaStream_t s);

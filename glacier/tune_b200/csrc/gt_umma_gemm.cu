@@ -1006,9 +1006,9 @@ cudaError_t umma_init_weight_maps(WeightDev *w, const char **err) {
         ok = ok && encode_2d(&w->tm_blk_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
                              (uint64_t)w->row_bytes, bb, 64, CU_TENSOR_MAP_SWIZZLE_NONE);
     }
-    if (w->qtype == kTypeQ4K)      // whole packed rows for the few-token streaming kernel
-        ok = ok && encode_2d(&w->tm_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, w->data, (uint64_t)w->row_bytes / 4, (uint64_t)w->N,
-                             (uint64_t)w->row_bytes, 72, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
+    // whole packed super-blocks of 16 rows for the few-token streaming kernel: two Q4_K blocks or one Q6_K block per row
+    ok = ok && encode_2d(&w->tm_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, w->data, (uint64_t)w->row_bytes / 4, (uint64_t)w->N,
+                         (uint64_t)w->row_bytes, w->qtype == kTypeQ4K ? 72 : 56, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (!ok) {
         if (err) *err = "cuTensorMapEncodeTiled failed for a weight tensor";
         return cudaErrorInvalidValue;
