@@ -19,6 +19,8 @@
 #include <cuda_fp16.h>
 
 #include "gt_engine_priv.h"
+#include "gt_mma.cuh"
+#include "gt_ptx.cuh"
 
 using namespace gt;
 
@@ -200,6 +202,111 @@ int ce_reserve(gt_engine *e, int T, int H, int vocab, bool want_grad, CeBuffers 
     return GT_OK;
 }
 
+// ------------------------------------------------------------------------------------------------
+// Logits of a few positions (up to 16): logits[T, V] = X[T, H] W[V, H]^T over fp16 rows.  Bound by reading W once from HBM
+// (1.09 GB for [152064, 3584]); the 128-row tcgen05 kernel, one launch per vocabulary tile, leaves a ramp of its own in
+// each of nine launches.  Here a block of 8 warps walks 16-row tiles with a stride of the grid; its warps split the
+// contraction, so the whole block waits for one memory latency per tile while the other resident blocks stream.  A thread
+// loads 16 bytes of rows g and g + 8 per 32 columns: with the contraction permuted alike on both sides these are the A
+// fragments of two m16n8k16 MMAs (fp16 operands, fp32 sums, as in the large kernel).  X is rounded to fp16 once per block.
+// ------------------------------------------------------------------------------------------------
+constexpr int kLogitsMaxT = 16, kLogitsWarps = 8;
+template <int NT>
+__global__ void __launch_bounds__(32 * kLogitsWarps) k_logits_few(const __half *__restrict__ W, const float *__restrict__ X, float *__restrict__ logits,
+                                                                 int T, int V, int H) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int xld = H * 2 + 16;                                   // rows 16 bytes apart modulo 128: conflict-free
+    __half *zero = reinterpret_cast<__half *>(smem + T * xld);    // 64 zero bytes, for columns beyond the tokens
+    float *red = reinterpret_cast<float *>(smem + T * xld + 64);  // [2][warps][16 rows][8 NT tokens]
+    constexpr int kRed = kLogitsWarps * 16 * 8 * NT;
+    pdl_wait();
+    pdl_trigger();
+    if (tid < 32) zero[tid] = __float2half_rn(0.f);
+    for (int i = tid; i < T * (H >> 2); i += 32 * kLogitsWarps) {
+        const int t = i / (H >> 2), c = i - t * (H >> 2);
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(X + (int64_t)t * H) + c);
+        const __half2 lo = __floats2half2_rn(v.x, v.y), hi = __floats2half2_rn(v.z, v.w);
+        *reinterpret_cast<uint2 *>(smem + t * xld + c * 8) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+    }
+    __syncthreads();
+    const int n32 = H >> 5;                                       // runs of 32 columns
+    const int r0 = n32 * warp / kLogitsWarps, r1 = n32 * (warp + 1) / kLogitsWarps;
+    const uint8_t *xrow[NT];
+    int xstep[NT];
+#pragma unroll
+    for (int n = 0; n < NT; n++) {
+        const bool live = n * 8 + g < T;
+        xrow[n] = live ? smem + (n * 8 + g) * xld + t4 * 16 : reinterpret_cast<const uint8_t *>(zero);
+        xstep[n] = live ? 64 : 0;
+    }
+    const int n_tiles = (V + 15) >> 4;
+    int buf = 0;
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, buf ^= 1) {
+        const int ra = min(tile * 16 + g, V - 1), rb = min(tile * 16 + g + 8, V - 1);
+        const uint4 *pa = reinterpret_cast<const uint4 *>(W + (int64_t)ra * H) + t4, *pb = reinterpret_cast<const uint4 *>(W + (int64_t)rb * H) + t4;
+        float acc[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+        constexpr int U = 7;      // 14 loads of 16 bytes in flight per thread
+        for (int r = r0; r < r1; r += U) {
+            uint4 a[U], b[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                a[u] = b[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (r + u < r1) {
+                    a[u] = __ldcs(pa + (r + u) * 4);
+                    b[u] = __ldcs(pb + (r + u) * 4);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if (r + u >= r1) break;
+                const uint32_t A0[4] = {a[u].x, b[u].x, a[u].y, b[u].y}, A1[4] = {a[u].z, b[u].z, a[u].w, b[u].w};
+#pragma unroll
+                for (int n = 0; n < NT; n++) {
+                    const uint4 x = *reinterpret_cast<const uint4 *>(xrow[n] + (r + u) * xstep[n]);
+                    mma16<__half>(acc[n], A0, x.x, x.y);
+                    mma16<__half>(acc[n], A1, x.z, x.w);
+                }
+            }
+        }
+        float *rd = red + buf * kRed;
+#pragma unroll
+        for (int n = 0; n < NT; n++) {
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                *reinterpret_cast<float2 *>(rd + (warp * 16 + g + 8 * h) * 8 * NT + n * 8 + 2 * t4) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+        }
+        __syncthreads();      // (the other buffer's readers are past the previous barrier's tile by the next one)
+        for (int i = tid; i < 16 * T; i += 32 * kLogitsWarps) {
+            const int row = i & 15, t = i >> 4;
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < kLogitsWarps; w++) v += rd[(w * 16 + row) * 8 * NT + t];
+            if (tile * 16 + row < V) logits[(int64_t)t * V + tile * 16 + row] = v;
+        }
+    }
+}
+
+template <int NT>
+cudaError_t launch_logits_nt(gt_engine *e, const WeightDev &wd, const float *hidden, float *logits, int T) {
+    static PerDeviceOnce configured;
+    const size_t smem = (size_t)T * (wd.K * 2 + 16) + 64 + 2 * kLogitsWarps * 16 * 8 * NT * sizeof(float);
+    cudaError_t ce = per_device_once(configured, [] { return cudaFuncSetAttribute(k_logits_few<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
+    if (ce != cudaSuccess) return ce;
+    // as many blocks as stay resident, walking the tiles together
+    int per_sm = 1;
+    ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_logits_few<NT>, 32 * kLogitsWarps, smem);
+    if (ce != cudaSuccess) return ce;
+    const int tiles = (wd.N + 15) / 16, grid = per_sm * e->sm_count < tiles ? per_sm * e->sm_count : tiles;
+    return launch_k(k_logits_few<NT>, dim3(grid), dim3(32 * kLogitsWarps), smem, e->stream, (const __half *)wd.data, hidden, logits, T, wd.N, wd.K);
+}
+// few positions, float4-aligned hidden rows, X beside the sums in shared memory
+bool logits_few_ok(const WeightDev &wd, const float *hidden, int T) {
+    return T <= kLogitsMaxT && wd.K % 32 == 0 && (reinterpret_cast<uintptr_t>(hidden) & 15) == 0 && (size_t)T * (wd.K * 2 + 16) <= 160 * 1024;
+}
+
 UmmaLaunch head_launch(gt_engine *e, const WeightDev *w, bool backward, const void *act16, int ld_act, int T, float *out, int ld_out,
                        int v0, int rows) {
     UmmaLaunch L;
@@ -331,6 +438,10 @@ int gt_lm_head_logits(gt_engine *e, const gt_weight *w, const float *hidden, flo
     if (V % 4 != 0) return failf(GT_ERR_UNSUPPORTED, "gt_lm_head_logits: vocabulary size must be a multiple of 4");
     std::lock_guard<std::mutex> lk(e->mu);
     GT_CUDA(cudaSetDevice(e->device));
+    if (logits_few_ok(wd, hidden, T)) {
+        GT_LAUNCH(e, T <= 8 ? launch_logits_nt<1>(e, wd, hidden, logits, T) : launch_logits_nt<2>(e, wd, hidden, logits, T));
+        return GT_OK;
+    }
     CeBuffers b;
     rc = ce_reserve(e, T, H, V, false, &b);
     if (rc != GT_OK) return rc;
