@@ -854,6 +854,17 @@ HostSlot &next_slot(gt_engine *e) {
     return sl;
 }
 
+// Copies of host-buffer calls on the two copy streams.  Asynchronous calls hand over page-locked buffers and must not block;
+// synchronous ones may hand over anything, and pageable memory goes through the copier's page-locked ring.
+cudaError_t upload(gt_engine *e, void *dst, const void *src, size_t bytes, int flags) {
+    if (flags & GT_FLAG_HOST_ASYNC) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, e->s_h2d);
+    return e->copier.to_device(dst, src, bytes, e->s_h2d);
+}
+cudaError_t download(gt_engine *e, void *dst, const void *src, size_t bytes, int flags) {
+    if (flags & GT_FLAG_HOST_ASYNC) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, e->s_d2h);
+    return e->copier.to_host(dst, src, bytes, e->s_d2h);
+}
+
 // A synchronous call returns with its outputs in the host buffers; an asynchronous one (pinned buffers) returns
 // once everything is queued, and gt_sync() completes it.
 int finish_host_call(gt_engine *e, int flags) {
@@ -876,7 +887,7 @@ int forward_host(gt_engine *e, int n, const gt_weight *const *w, gt_adapter *con
         Yd[j] = (float *)sl.out[j].p;
     }
     if (sl.used) GT_CUDA(cudaStreamWaitEvent(e->s_h2d, sl.compute_done, 0));      // the slot's last call has read its inputs
-    GT_CUDA(cudaMemcpyAsync(sl.in[0].p, X, bx, cudaMemcpyHostToDevice, e->s_h2d));
+    GT_CUDA(upload(e, sl.in[0].p, X, bx, flags));
     GT_CUDA(cudaEventRecord(sl.h2d_done, e->s_h2d));
     GT_CUDA(cudaStreamWaitEvent(e->stream, sl.h2d_done, 0));
     if (sl.used) GT_CUDA(cudaStreamWaitEvent(e->stream, sl.d2h_done, 0));         // ... and its outputs have left
@@ -894,8 +905,7 @@ int forward_host(gt_engine *e, int n, const gt_weight *const *w, gt_adapter *con
     }
     GT_CUDA(cudaEventRecord(sl.compute_done, e->stream));
     GT_CUDA(cudaStreamWaitEvent(e->s_d2h, sl.compute_done, 0));
-    for (int j = 0; j < n; j++)
-        GT_CUDA(cudaMemcpyAsync(Y[j], Yd[j], (size_t)T * w[j]->dev.N * sizeof(float), cudaMemcpyDeviceToHost, e->s_d2h));
+    for (int j = 0; j < n; j++) GT_CUDA(download(e, Y[j], Yd[j], (size_t)T * w[j]->dev.N * sizeof(float), flags));
     GT_CUDA(cudaEventRecord(sl.d2h_done, e->s_d2h));
     sl.used = true;
     return finish_host_call(e, flags);
@@ -928,11 +938,10 @@ int backward_host(gt_engine *e, int n, const gt_weight *const *w, gt_adapter *co
         GT_CUDA(cudaStreamWaitEvent(e->s_h2d, sl.compute_done, 0));
         if (dX && !assign) GT_CUDA(cudaStreamWaitEvent(e->s_h2d, sl.d2h_done, 0));
     }
-    for (int j = 0; j < n; j++)
-        GT_CUDA(cudaMemcpyAsync(sl.in[j].p, dY[j], (size_t)T * w[j]->dev.N * sizeof(float), cudaMemcpyHostToDevice, e->s_h2d));
-    if (need_x) GT_CUDA(cudaMemcpyAsync(sl.in[kSlotIn - 1].p, X, bx, cudaMemcpyHostToDevice, e->s_h2d));
+    for (int j = 0; j < n; j++) GT_CUDA(upload(e, sl.in[j].p, dY[j], (size_t)T * w[j]->dev.N * sizeof(float), flags));
+    if (need_x) GT_CUDA(upload(e, sl.in[kSlotIn - 1].p, X, bx, flags));
     // "dX +=": the reference uploads dX too and the kernel accumulates into it (GpuLoraEngine.Backward.cs:85-89)
-    if (dX && !assign) GT_CUDA(cudaMemcpyAsync(sl.out[0].p, dX, bx, cudaMemcpyHostToDevice, e->s_h2d));
+    if (dX && !assign) GT_CUDA(upload(e, sl.out[0].p, dX, bx, flags));
     GT_CUDA(cudaEventRecord(sl.h2d_done, e->s_h2d));
     GT_CUDA(cudaStreamWaitEvent(e->stream, sl.h2d_done, 0));
     if (sl.used) GT_CUDA(cudaStreamWaitEvent(e->stream, sl.d2h_done, 0));
@@ -941,7 +950,7 @@ int backward_host(gt_engine *e, int n, const gt_weight *const *w, gt_adapter *co
     if (rc != GT_OK) return rc;
     GT_CUDA(cudaEventRecord(sl.compute_done, e->stream));
     GT_CUDA(cudaStreamWaitEvent(e->s_d2h, sl.compute_done, 0));
-    if (dX) GT_CUDA(cudaMemcpyAsync(dX, sl.out[0].p, bx, cudaMemcpyDeviceToHost, e->s_d2h));
+    if (dX) GT_CUDA(download(e, dX, sl.out[0].p, bx, flags));
     GT_CUDA(cudaEventRecord(sl.d2h_done, e->s_d2h));
     sl.used = true;
     return finish_host_call(e, flags);
@@ -1522,7 +1531,7 @@ int gt_ffn_forward(gt_engine *e, const gt_weight *w_gate, const gt_weight *w_up,
         }
     }
     if (sl.used) GT_CUDA(cudaStreamWaitEvent(e->s_h2d, sl.compute_done, 0));
-    GT_CUDA(cudaMemcpyAsync(sl.in[0].p, X, bx, cudaMemcpyHostToDevice, e->s_h2d));
+    GT_CUDA(upload(e, sl.in[0].p, X, bx, flags));
     GT_CUDA(cudaEventRecord(sl.h2d_done, e->s_h2d));
     GT_CUDA(cudaStreamWaitEvent(e->stream, sl.h2d_done, 0));
     if (sl.used) GT_CUDA(cudaStreamWaitEvent(e->stream, sl.d2h_done, 0));
@@ -1530,9 +1539,9 @@ int gt_ffn_forward(gt_engine *e, const gt_weight *w_gate, const gt_weight *w_up,
     if (rc != GT_OK) return rc;
     GT_CUDA(cudaEventRecord(sl.compute_done, e->stream));
     GT_CUDA(cudaStreamWaitEvent(e->s_d2h, sl.compute_done, 0));
-    GT_CUDA(cudaMemcpyAsync(out_down, sl.out[0].p, bx, cudaMemcpyDeviceToHost, e->s_d2h));
+    GT_CUDA(download(e, out_down, sl.out[0].p, bx, flags));
     for (int i = 0; i < 3; i++)
-        if (host_out[i]) GT_CUDA(cudaMemcpyAsync(host_out[i], dev_out[i], bf, cudaMemcpyDeviceToHost, e->s_d2h));
+        if (host_out[i]) GT_CUDA(download(e, host_out[i], dev_out[i], bf, flags));
     GT_CUDA(cudaEventRecord(sl.d2h_done, e->s_d2h));
     sl.used = true;
     return finish_host_call(e, flags);

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../../include/glaciertune_b200.h"
+#include "gt_hostcopy.h"
 #include "gt_internal.h"
 #include "gt_quant.cuh"
 
@@ -96,6 +97,7 @@ struct gt_engine {
     // synchronous call still overlaps its own download with nothing in its way.
     HostSlot slots[kHostSlots];
     int slot_next = 0;
+    gt::HostCopier copier;       // pageable host buffers of the synchronous calls
     cudaStream_t s_h2d = nullptr, s_d2h = nullptr;
     // overlapped gradient exchange: collectives queued on a side stream between a fork and a join of the engine stream
     cudaStream_t s_comm = nullptr;
