@@ -90,6 +90,13 @@ __device__ __forceinline__ void tma_prefetch_desc(const void *tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 
+// one lane of a converged warp (the same one every time)
+__device__ __forceinline__ bool elect_one() {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+    return ok != 0;
+}
+
 // ---------------------------------------------------------------- tcgen05 / TMEM
 // Whole-warp calls (.sync.aligned).
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {

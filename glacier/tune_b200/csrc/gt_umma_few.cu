@@ -206,8 +206,11 @@ __global__ void __launch_bounds__(kThreadsF, 1) k_umma_few(const __grid_constant
         }
     } else if (warp == 1 || warp == kIssuer2) {
         // ------------------------------------------------------------------ two independent MMA issuers
-        if (lane == 0) {
+        // (the whole warp walks the loop, one elected lane issues: see gt_umma_gemm.cu)
+        {
             const int who = warp == 1 ? 0 : 1;
+            const bool el = elect_one();
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             bool ok = true;
             // descriptors as (lo, hi) words: lo = (addr >> 4) | (LBO >> 4) << 16, hi = (SBO >> 4) | version 1 << 14 | layout << 29
             constexpr uint32_t kHi64 = (512u >> 4) | (1u << 14) | (4u << 29);        // K-major, 64-byte swizzle
@@ -216,25 +219,29 @@ __global__ void __launch_bounds__(kThreadsF, 1) k_umma_few(const __grid_constant
             constexpr uint32_t kBLoField = (BWD ? (4096u >> 4) : 1u) << 16;          // MN-major: LBO = stride between 64-column images
             constexpr uint32_t kBStep = (BWD ? 2048u : 32u) >> 4;                    // per k-step advance of the B operand
             const uint32_t idesc = umma_idesc_f16(kFmt, 0u, BWD ? 1u : 0u, (uint32_t)kTileN, (uint32_t)kTok);
-            const uint32_t d_tmem = tmem_base + (uint32_t)(who * kTileN);
+            const uint32_t d_tmem = tmem_u + (uint32_t)(who * kTileN);
             for (int n = who; n < n_total && ok; n += 2) {
                 const int si = n % kSlots, m = n >> 1, xi = m % kXSlots;
                 ok = mbar_wait_bounded(bar(kBXFull + xi), (uint32_t)(m / kXSlots) & 1u, abort_flag, p.status, kFewMma + 2);
-                if (!ok) break;
-                ok = mbar_wait_bounded(bar(kBFull + si), (uint32_t)(n / kSlots) & 1u, abort_flag, p.status, kFewMma + 1);
+                ok = ok && mbar_wait_bounded(bar(kBFull + si), (uint32_t)(n / kSlots) & 1u, abort_flag, p.status, kFewMma + 1);
+                ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after_sync();
-                if (who == 0) trace(8, n >> 1);
+                if (who == 0 && el) trace(8, n >> 1);
                 // this issuer's half of the activation tile: k-steps 2 who, 2 who + 1 of its 128-byte rows
                 const uint32_t a_lo = (((sbase + kOffXf + xi * kXSlotBytes) & 0x3FFFFu) >> 4) + (uint32_t)(who * 4) | (1u << 16);
                 const uint32_t b_lo = (((sbase + kOffWf + si * kWSlotBytes) & 0x3FFFFu) >> 4) | kBLoField;
-                umma_f16_ss_lohi<false>(d_tmem, a_lo, kHi128, b_lo, kBHi, idesc, n == who ? 0u : 1u);
-                umma_f16_ss_lohi<false>(d_tmem, a_lo + 2, kHi128, b_lo + kBStep, kBHi, idesc, 1u);
-                umma_commit(bar(kBEmpty + si));
-                umma_commit(bar(kBXEmpty + xi));
-                if (who == 0) trace(9, n >> 1);
+                if (el) {
+                    umma_f16_ss_lohi<false>(d_tmem, a_lo, kHi128, b_lo, kBHi, idesc, n == who ? 0u : 1u);
+                    umma_f16_ss_lohi<false>(d_tmem, a_lo + 2, kHi128, b_lo + kBStep, kBHi, idesc, 1u);
+                    umma_commit(bar(kBEmpty + si));
+                    umma_commit(bar(kBXEmpty + xi));
+                }
+                __syncwarp();
+                if (who == 0 && el) trace(9, n >> 1);
             }
-            if (ok) umma_commit(bar(kBAcc));
+            if (ok && el) umma_commit(bar(kBAcc));
+            __syncwarp();
         }
     } else {
         // ------------------------------------------------------------------ dequant warps, then epilogue

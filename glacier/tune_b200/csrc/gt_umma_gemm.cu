@@ -128,6 +128,29 @@ struct Ring {
     }
 };
 
+// 32 columns of a lane's accumulator row -> 32 tokens of its output column (the first n of them).  Whether to add and whether
+// the chunk is whole is decided once, not per element: with both tests inside the loop a warp issued one 128-byte store per
+// 83 clocks.
+__device__ __forceinline__ void store_chunk(const uint32_t (&v)[32], float *dst, int ld, int n, bool add, float bias) {
+    if (n >= 32) {
+        if (add) {
+#pragma unroll
+            for (int j = 0; j < 32; j++, dst += ld) atomicAdd(dst, __uint_as_float(v[j]));
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; j++, dst += ld) *dst = __uint_as_float(v[j]) + bias;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j++, dst += ld) {
+            if (j < n) {
+                if (add) atomicAdd(dst, __uint_as_float(v[j]));
+                else *dst = __uint_as_float(v[j]) + bias;
+            }
+        }
+    }
+}
+
 // PAIR = false: one CTA per tile, tcgen05 cta_group::1, M = 128.
 // PAIR = true : a cluster of two CTAs (the two SMs of a TPC) works on two adjacent tiles with cta_group::2 MMAs of
 //               M = 256.  Each CTA dequantizes its own 128 weight rows and loads only HALF of the token rows of
@@ -439,8 +462,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
         // a fence and a commit: two threads take alternate stages, so one waits for its next stage while the other
         // keeps the pipe fed.  They hand a turn token back and forth, so stages are queued in order and the fp32
         // accumulation order does not change from run to run.  tcgen05.commit tracks the MMAs of the committing thread, so each releases its own stages.
-        if (lane == 0 && leader) {
+        // The whole warp walks the loop and one elected lane issues: with warp-uniform control flow the descriptors live in
+        // uniform registers.  (Inside `if (lane == 0)` every operand was moved there MMA by MMA: 85 clocks per MMA of one
+        // issuing thread against 39, and about 300 clocks between a commit and the next stage's first MMA.)
+        if (leader) {
             const int who = warp == 1 ? 0 : 1;
+            const bool el = elect_one();
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             bool ok = true;
             const uint32_t a_mn = BWD ? 1u : 0u;
             auto wait_full = [&](int n, int code) -> bool {
@@ -449,7 +477,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                 const bool r = PAIR ? mbar_wait_bounded_cluster(bar(slot), phase, abort_flag, p.status, code)
                                     : mbar_wait_bounded(bar(slot), phase, abort_flag, p.status, code);
                 tc_fence_after_sync();
-                return r;
+                return __all_sync(0xffffffffu, r);
             };
             const int n_main = (u1 - u0) * kSub;
             const int n_total = n_main + n_lora;
@@ -478,42 +506,47 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                     // its own operands, which is the latency the second issuer hides)
                     const uint32_t turn_phase = (uint32_t)(who == 1 ? (n >> 1) : ((n >> 1) - 1)) & 1u;
                     ok = mbar_wait_bounded(bar(kBarTurn + who), turn_phase, abort_flag, p.status, kCodeMma + 5);
+                    ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                 }
-                if (who == 0) trace(8, n);
+                if (who == 0 && el) trace(8, n);
                 const uint32_t first = n == (par ? who : 0) ? 0u : 1u;     // the very first MMA into an accumulator overwrites it
-                // k-step-major order: consecutive MMAs alternate between the accumulators (measured faster than
-                // finishing one accumulator's k-steps first)
+                if (el) {
+                    // k-step-major order: consecutive MMAs alternate between the accumulators (measured faster than
+                    // finishing one accumulator's k-steps first)
 #pragma unroll
-                for (int ks = 0; ks < 4; ks++) {
-                    if (ks < ksteps) {
-                        const uint32_t a_lo = a_lo0 + ks * kAStep;
-                        if (PAIR && n_mma > 1) {
+                    for (int ks = 0; ks < 4; ks++) {
+                        if (ks < ksteps) {
+                            const uint32_t a_lo = a_lo0 + ks * kAStep;
+                            if (PAIR && n_mma > 1) {
 #pragma unroll
-                            for (int i = 0; i < kMaxMma; i++)
-                                if (i < n_mma)
-                                    umma_f16_ss_lohi<true>(tmem_base + i * MTOK, a_lo, kDescHi, b_lo0 + i * (kMmaSlotBytes >> 4) + ks * 2,
-                                                           kDescHi, idesc[i], ks == 0 ? first : 1u);
-                        } else if (PAIR) {
-                            // one MMA per k-step (tokens <= MTOK): each k-step into its own partial accumulator
-                            const int a = ks % n_acc;
-                            umma_f16_ss_lohi<true>(tmem_base + a * acc_stride, a_lo, kDescHi, b_lo0 + ks * 2, kDescHi, idesc[0],
-                                                   ks < n_acc ? first : 1u);
-                        } else {
-                            // few tokens: one MMA per k-step, each k-step into its own partial accumulator
-                            const int a = (par ? who * n_acc_per : 0) + ks % n_acc_per;
-                            umma_f16_ss_lohi<false>(tmem_base + a * acc_stride, a_lo, kDescHi, b_lo0 + ks * 2, kDescHi, idesc[0],
-                                                    ks < n_acc_per ? first : 1u);
+                                for (int i = 0; i < kMaxMma; i++)
+                                    if (i < n_mma)
+                                        umma_f16_ss_lohi<true>(tmem_u + i * MTOK, a_lo, kDescHi, b_lo0 + i * (kMmaSlotBytes >> 4) + ks * 2,
+                                                               kDescHi, idesc[i], ks == 0 ? first : 1u);
+                            } else if (PAIR) {
+                                // one MMA per k-step (tokens <= MTOK): each k-step into its own partial accumulator
+                                const int a = ks % n_acc;
+                                umma_f16_ss_lohi<true>(tmem_u + a * acc_stride, a_lo, kDescHi, b_lo0 + ks * 2, kDescHi, idesc[0],
+                                                       ks < n_acc ? first : 1u);
+                            } else {
+                                // few tokens: one MMA per k-step, each k-step into its own partial accumulator
+                                const int a = (par ? who * n_acc_per : 0) + ks % n_acc_per;
+                                umma_f16_ss_lohi<false>(tmem_u + a * acc_stride, a_lo, kDescHi, b_lo0 + ks * 2, kDescHi, idesc[0],
+                                                        ks < n_acc_per ? first : 1u);
+                            }
                         }
                     }
+                    if (PAIR) umma_commit_pair(bar(kBarEmpty + si)); else umma_commit(bar(kBarEmpty + si));
+                    if (!par) mbar_arrive(bar(kBarTurn + (who ^ 1)));
                 }
-                if (PAIR) umma_commit_pair(bar(kBarEmpty + si)); else umma_commit(bar(kBarEmpty + si));
-                if (!par) mbar_arrive(bar(kBarTurn + (who ^ 1)));
-                if (who == 0) trace(9, n);
+                __syncwarp();
+                if (who == 0 && el) trace(9, n);
             }
-            if (ok) {
+            if (ok && el) {
                 if (PAIR) umma_commit_pair(bar(kBarAcc)); else umma_commit(bar(kBarAcc));
             }
+            __syncwarp();
         }
     } else {
         // ------------------------------------------------------------------ dequant warps, then epilogue
@@ -817,19 +850,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
 #pragma unroll
                     for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w2[j]));
                 }
-                if (row_ok) {
-#pragma unroll
-                    for (int j = 0; j < 32; j++) {
-                        const int tl = c * 32 + j;
-                        const int t = tok0 + tl;
-                        if (tl < tb && t < p.T) {
-                            float *dst = out_base + (int64_t)t * ld_out + orow;
-                            const float val = __uint_as_float(v[j]);
-                            if (p.atomic_out) atomicAdd(dst, val);
-                            else *dst = val + bv;       // this CTA alone owns the tile (backward: bv is 0)
-                        }
-                    }
-                }
+                if (row_ok) store_chunk(v, out_base + (int64_t)(tok0 + c * 32) * ld_out + orow, ld_out, min(tb, p.T - tok0) - c * 32, p.atomic_out != 0, bv);
             }
         }
     }
