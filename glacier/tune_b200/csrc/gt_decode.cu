@@ -820,7 +820,7 @@ bool decode_group_ok(const WeightDev *const *w, int n, bool dual, int T, int sm_
     if (T < 1 || T > stream_max_tokens() || n < 1 || n > kMaxMembers) return false;
     int units = 0;
     for (int j = 0; j < n; j++) {
-        if ((w[j]->qtype != kTypeQ4K && w[j]->qtype != kTypeQ6K) || !w[j]->tma_ok || w[j]->K != w[0]->K) return false;
+        if ((w[j]->qtype != kTypeQ4K && w[j]->qtype != kTypeQ6K) || !w[j]->tma_ok || w[j]->pair_hb || w[j]->K != w[0]->K) return false;
         if (!dual || j == 0) units += (w[j]->N + 15) / 16;
     }
     return plan(T, w[0]->K, units, dual ? 2 : 1, sm_count).S > 0;

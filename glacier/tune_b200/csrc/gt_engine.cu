@@ -354,98 +354,31 @@ int forward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adap
 }
 
 // out[T, N] = act * W^T (+bias) (+ lora) on the engine stream, device pointers.
-// the base product of a paired-row tensor on the tensor path (see the paired-row kernels in gt_fp32_kernels.cu)
-bool paired_path(const gt_engine *e, const gt_weight *w) { return e->math_mode != GT_MATH_FP32 && w->has_paired; }
-
-int paired_forward_base(gt_engine *e, const gt_weight *w, const float *Xd, float *Yd, int T) {
-    const WeightDev &wd = w->dev, &pv = w->paired;
-    const int fp16 = e->math_mode == GT_MATH_FP16;
-    GT_CUDA(e->x16.reserve((size_t)2 * T * pv.K * 2));
-    GT_CUDA(e->pair_tmp.reserve((size_t)2 * T * pv.N * sizeof(float)));
-    GT_LAUNCH(e, launch_pair_expand16(Xd, e->x16.p, T, wd.K, fp16, e->stream));
-    UmmaLaunch L;
-    L.w = &pv;
-    L.fp16 = fp16;
-    L.act16 = e->x16.p;
-    L.ld_act = pv.K;
-    L.T = 2 * T;
-    L.out = (float *)e->pair_tmp.p;
-    L.ld_out = pv.N;
-    L.status = e->status;
-    L.trace = e->trace;
-    L.splits = umma_group_splits(&L, 1, e->sm_count);
-    if (L.splits > 1) {
-        GT_LAUNCH(e, launch_fill_rows(L.out, nullptr, 2 * T, pv.N, e->stream));
-        L.out_prefilled = 1;
-    }
-    const char *msg = nullptr;
-    cudaError_t ce = timed_umma_group(e, &L, 1, &msg);
-    if (ce != cudaSuccess) return fail(GT_ERR_CUDA, "forward GEMM launch failed: %s", msg ? msg : cudaGetErrorString(ce));
-    GT_LAUNCH(e, launch_pair_interleave(L.out, wd.bias, Yd, T, wd.N, e->stream));
-    return GT_OK;
-}
-
-int paired_backward_base(gt_engine *e, const gt_weight *w, const float *dYd, float *dXd, int T, bool assign) {
-    const WeightDev &wd = w->dev, &pv = w->paired;
-    const int fp16 = e->math_mode == GT_MATH_FP16;
-    const int ld16 = round8(pv.N);
-    GT_CUDA(e->dy16.reserve((size_t)2 * T * ld16 * 2));
-    GT_CUDA(e->pair_tmp.reserve((size_t)2 * T * pv.K * sizeof(float)));
-    GT_LAUNCH(e, launch_pair_gather16(dYd, e->dy16.p, T, wd.N, ld16, fp16, e->stream));
-    UmmaLaunch L;
-    L.w = &pv;
-    L.backward = 1;
-    L.fp16 = fp16;
-    L.act16 = e->dy16.p;
-    L.ld_act = ld16;
-    L.T = 2 * T;
-    L.out = (float *)e->pair_tmp.p;
-    L.ld_out = pv.K;
-    L.status = e->status;
-    L.trace = e->trace;
-    L.splits = umma_group_splits(&L, 1, e->sm_count);
-    if (L.splits == 1) L.out_assign = 1;
-    else GT_LAUNCH(e, launch_fill_rows(L.out, nullptr, 2 * T, pv.K, e->stream));
-    const char *msg = nullptr;
-    cudaError_t ce = timed_umma_group(e, &L, 1, &msg);
-    if (ce != cudaSuccess) return fail(GT_ERR_CUDA, "backward GEMM launch failed: %s", msg ? msg : cudaGetErrorString(ce));
-    GT_LAUNCH(e, launch_pair_fold(L.out, dXd, T, wd.K, assign ? 1 : 0, e->stream));
-    return GT_OK;
-}
-
 int forward_device(gt_engine *e, const gt_weight *w, gt_adapter *ad, const float *Xd, float *Yd, int T, bool use_lora) {
     if (tensor_path(e, w)) return forward_group_device(e, 1, &w, &ad, Xd, &Yd, T, use_lora ? 0 : GT_FLAG_NO_LORA);
     const WeightDev &wd = w->dev;
     const int N = wd.N, K = wd.K;
-    if (paired_path(e, w)) {
-        int prc = paired_forward_base(e, w, Xd, Yd, T);
-        if (prc != GT_OK) return prc;
-    }
     if (use_lora) {
         int rc = compute_low(e, &ad, 1, Xd, nullptr, 0, T, K);
         if (rc != GT_OK) return rc;
     }
-    if (!paired_path(e, w)) {
-        ExactGemm g;
-        g.qtype = wd.qtype;
-        g.w = wd.data;
-        g.act = Xd;
-        g.out = Yd;
-        g.bias = wd.bias;
-        g.T = T;
-        g.N = N;
-        g.K = K;
-        if (use_lora) {
-            g.lora_act = low_of(ad);
-            g.lora_w = ad->B;
-            g.scale = ad->scaling;
-            g.R = ad->rank;
-            g.flag = ad->b_nonzero;
-        }
-        GT_LAUNCH(e, launch_exact_gemm(g, e->sm_count, e->stream));
-    } else if (use_lora) {
-        GT_LAUNCH(e, launch_lora_delta_fp32(low_of(ad), ad->B, Yd, nullptr, T, N, ad->rank, ad->scaling, ad->b_nonzero, e->stream));
+    ExactGemm g;
+    g.qtype = wd.qtype;
+    g.w = wd.data;
+    g.act = Xd;
+    g.out = Yd;
+    g.bias = wd.bias;
+    g.T = T;
+    g.N = N;
+    g.K = K;
+    if (use_lora) {
+        g.lora_act = low_of(ad);
+        g.lora_w = ad->B;
+        g.scale = ad->scaling;
+        g.R = ad->rank;
+        g.flag = ad->b_nonzero;
     }
+    GT_LAUNCH(e, launch_exact_gemm(g, e->sm_count, e->stream));
     if (!use_lora && ad) ad->low_T = 0;
     return GT_OK;
 }
@@ -653,20 +586,14 @@ int backward_device(gt_engine *e, const gt_weight *w, gt_adapter *ad, const floa
     // exact fp32 kernels (validation mode, weights outside the tensor-core layout) or adapter gradients only
     const WeightDev &wd = w->dev;
     const int N = wd.N, K = wd.K;
-    const bool paired = paired_path(e, w) && dXd;
-    if (paired) {      // the base product writes (or adds into) dX itself
-        int prc = paired_backward_base(e, w, dYd, dXd, T, assign);
-        if (prc != GT_OK) return prc;
-    }
     if (use_lora) {
         const bool lora = true;
         void *no16 = nullptr;
         const int ld16 = round8(N);
         int rc = lora_backward_group(e, 1, &w, &ad, &lora, &dYd, Xd, &no16, &ld16, T, reuse_low, nullptr);
         if (rc != GT_OK) return rc;
-        if (paired) GT_LAUNCH(e, launch_lora_dx_fp32(dlow_of(ad, T), ad->A, dXd, ad->scaling, T, K, ad->rank, e->stream));
     }
-    if (dXd && !paired) {
+    if (dXd) {
         ExactGemm g;
         g.qtype = wd.qtype;
         g.w = wd.data;
@@ -1058,7 +985,7 @@ int gt_engine_destroy(gt_engine *e) {
     if (e->stream) cudaStreamSynchronize(e->stream);
     if (e->s_h2d) cudaStreamSynchronize(e->s_h2d);
     if (e->s_d2h) cudaStreamSynchronize(e->s_d2h);
-    Scratch *all[] = {&e->x16, &e->dy16, &e->dlow, &e->ytmp, &e->pair_tmp, &e->ffn[0], &e->ffn[1], &e->ffn[2], &e->ce, &e->ce_host, &e->attn, &e->low_parts};
+    Scratch *all[] = {&e->x16, &e->dy16, &e->dlow, &e->ytmp, &e->ffn[0], &e->ffn[1], &e->ffn[2], &e->ce, &e->ce_host, &e->attn, &e->low_parts};
     for (Scratch *s : all) s->release();
     for (HostSlot &sl : e->slots) {
         for (Scratch &b : sl.in) b.release();
@@ -1221,18 +1148,8 @@ int gt_weight_upload(gt_engine *e, int ggml_type, const void *host_bytes, int64_
         gt_weight_free(w);
         return fail(GT_ERR_CUDA, "%s", msg ? msg : "tensor map creation failed");
     }
-    if (!d.tma_ok && (ggml_type == GT_TYPE_Q4_K || ggml_type == GT_TYPE_Q6_K) && in_features % 256 == 128 && out_features % 2 == 0) {
-        WeightDev &v = w->paired;
-        v = d;
-        v.bias = nullptr;
-        v.N = out_features / 2;
-        v.K = 2 * in_features;
-        v.row_bytes = (int64_t)(v.K / 256) * dev_block_bytes(ggml_type);
-        const char *pm = nullptr;
-        w->has_paired = umma_init_weight_maps(&v, &pm) == cudaSuccess && v.tma_ok;
-    }
     logf(GT_LOG_DEBUG, "weight [%d, %d] type %d uploaded: %.2f MB on device %d%s", out_features, in_features, ggml_type, (double)d.nbytes / 1e6,
-         e->device, d.tma_ok ? "" : (w->has_paired ? " (tensor path through the paired-row view)" : " (CUDA-core path only)"));
+         e->device, d.tma_ok ? "" : " (exact kernels only)");
     *out = w;
     return GT_OK;
 }

@@ -87,7 +87,7 @@ struct gt_engine {
     std::mutex mu;
     int *status = nullptr;       // device int[4]; [0] = first bounded-wait timeout code
     double *clip = nullptr;      // device double[2]
-    Scratch x16, dy16, dlow, ytmp, pair_tmp;
+    Scratch x16, dy16, dlow, ytmp;
     Scratch ce, ce_host;         // LM-head cross-entropy: logits / probability tiles and per-token state; host staging
     Scratch attn;                // attention: log-sum-exp rows and the dO.O row sums
     Scratch low_parts;           // partial sums of X*A of the few-token forward
@@ -123,10 +123,6 @@ struct gt_engine {
 struct gt_weight {
     gt_engine *eng = nullptr;
     gt::WeightDev dev;
-    // K-quant tensor with in_features % 256 == 128 and an even row count: the same bytes seen as [N / 2, 2 K], whole
-    // super-blocks per row, with tensor maps (shares dev.data; owns nothing)
-    gt::WeightDev paired;
-    bool has_paired = false;
 };
 
 struct gt_adapter {

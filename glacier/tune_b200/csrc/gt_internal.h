@@ -36,7 +36,8 @@ struct WeightDev {
     int64_t nbytes = 0;
     int64_t row_bytes = 0;        // K/256 * block bytes when K % 256 == 0, else 0 (flat super-block stream)
     float *bias = nullptr;        // [N] or null
-    bool tma_ok = false;          // row-aligned and tensor maps built
+    bool tma_ok = false;          // tensor maps built: rows of whole super-blocks, or pairs of rows
+    int pair_hb = 0;              // maps over pairs of rows (in_features % 256 == 128): half super-blocks per row, else 0
     CUtensorMap tm_hdr, tm_q0, tm_q1;   // 2-D byte maps over [N, row_bytes], boxes of 64 rows (backward raw stages)
     CUtensorMap tm_hdr_f, tm_q0_f, tm_q1_f;   // the same with boxes of 128 rows (forward raw stages: half as many copies)
     CUtensorMap tm_rows;                // 32-bit words over [N, row_bytes / 4], boxes of 16 rows x two Q4_K blocks / one Q6_K block
@@ -83,11 +84,6 @@ cudaError_t launch_lora_bwd_x(const float *X, const float *dLow, float *dA, floa
 cudaError_t launch_lora_dx_fp32(const float *dLow, const float *A, float *dX, float scaling, int T, int K, int R,
                                 cudaStream_t s);
 cudaError_t launch_cast16(const float *src, void *dst, int rows, int cols, int ld_dst, int fp16, cudaStream_t s);
-// paired-row view of a tensor with in_features % 256 == 128 (see gt_fp32_kernels.cu)
-cudaError_t launch_pair_expand16(const float *X, void *x2, int T, int K, int fp16, cudaStream_t s);
-cudaError_t launch_pair_interleave(const float *tmp, const float *bias, float *Y, int T, int N, cudaStream_t s);
-cudaError_t launch_pair_gather16(const float *dY, void *dy2, int T, int N, int ld, int fp16, cudaStream_t s);
-cudaError_t launch_pair_fold(const float *Z, float *dX, int T, int K, int assign, cudaStream_t s);
 // Y[t, :] = bias (or 0)
 cudaError_t launch_fill_rows(float *Y, const float *bias, int T, int N, cudaStream_t s);
 // residual += Y

@@ -108,6 +108,9 @@ struct Params {
     // holds 64 rows of member 0 and the SAME 64 rows of member 1, laid out so that TMEM lanes 32 q + l and 32 q + 16 + l
     // (l < 16) are the two members' row 16 q + l: one warp shuffle brings gate and up of a feature together.
     int dual;
+    // Rows of an odd number of half super-blocks (in_features % 256 == 128): the byte stream is addressed as rows of two
+    // weight rows each (whole super-blocks again); weight row 2 s + h starts pair_hb * h half-blocks into row s.  0: plain rows
+    int pair_hb;
     void *h16;       // T16 [T, ld_h16]: SiLU(gate) * up, or null
     int ld_h16;
 };
@@ -371,14 +374,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                     }
                 }
             }
-        } else if (lane < ((!BWD && p.dual) ? 6 : 3) * kTeams) {
+        } else if (lane < ((p.pair_hb || (!BWD && p.dual)) ? 6 : 3) * kTeams) {
             // Teams of three lanes (lane 0 of a team arms the barrier and copies the headers, lanes 1 and 2 copy the
             // quant regions); team t issues the raw stages r = t (mod kTeams).  Issuing a tiled copy holds the issuing
             // thread for several hundred clocks: with one team the issue rate alone (one raw stage per ~800 clocks) paced
             // the few-token shapes.  kTeams <= kNumRaw, so a team never waits for a slot whose previous stage is issued
             // in the same round.
-            // (dual forward: six lanes, one per region and member)
-            const int lpt = (!BWD && p.dual) ? 6 : 3;
+            // (dual forward: six lanes, one per region and member; paired rows: one per region and row of a pair)
+            const int lpt = (p.pair_hb || (!BWD && p.dual)) ? 6 : 3;
             const int team = lane / lpt, li = lane - lpt * team;
             bool ok = true;
             for (int u = u0 + team; u < u1 && ok; u += kTeams) {
@@ -397,6 +400,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                     sb = u >> 1; half = u & 1; row0 = ltile * kTileW;
                 }
                 const Member &W = p.m[um];
+                if (p.pair_hb) {
+                    // half as many rows from either weight row of a pair: row h's boxes land behind row 0's in every region
+                    const int reg = li % 3, h = li / 3;
+                    const int hb = (BWD ? tile : u) + h * p.pair_hb, x = (hb >> 1) * QS::kBlockBytes, hf = hb & 1;
+                    const int region = reg == 0 ? 0 : (reg == 1 ? kRows * H : kRows * (H + 64));
+                    const int row_bytes = reg == 0 ? H : (reg == 1 ? 64 : Q1);
+                    if (li == 0) {
+                        mbar_arrive_expect_tx(rbar, (uint32_t)(kRows * (H + 64 + Q1)));
+                        if (lane == 0) trace(0, r / kTeams);
+                    }
+                    if (reg < 2 || Q1 > 0)
+                        tma_load_2d(rdst + region + h * (kRows / 2) * row_bytes, reg == 0 ? &W.tm_hdr : (reg == 1 ? &W.tm_q0 : &W.tm_q1),
+                                    x + (reg == 0 ? QS::hdr_x(hf) : (reg == 1 ? QS::q0_x(hf) : QS::q1_x(hf))), row0 >> 1, rbar);
+                    continue;
+                }
                 row0 += W.row_base;
                 const int xb = sb * QS::kBlockBytes;
                 if (!BWD && p.dual) {
@@ -567,7 +585,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
         };
         // operand stage n lives in A slot n % kNumA with phase (n / kNumA) & 1; raw stage i in slot i % kNumRaw.
         // Runs r = 0, 1 of this thread: 32-weight group grp[r] of the row, written at dst_off[r] + chunk0[r].
-        auto produce = [&](int n, const uint8_t *rs, int row, int half, const int (&grp)[2], const uint32_t (&dst_off)[2],
+        // (row: its row in the raw stage, swz: swizzle phase of its row in the operand tile)
+        auto produce = [&](int n, const uint8_t *rs, int row, int swz, int half, const int (&grp)[2], const uint32_t (&dst_off)[2],
                            const int (&chunk0)[2]) -> bool {
             const int ai = n % kNumA;
             if (!mbar_wait_bounded(bar(kBarEmpty + ai), ((uint32_t)(n / kNumA) & 1u) ^ 1u, abort_flag, p.status, kCodeDequant + 2))
@@ -578,7 +597,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
             for (int r = 0; r < 2; r++)
                 dequant32_to_swizzled_row<QT, T16>(rs + row * H, rs + kRows * H + row * 64,
                                                    rs + kRows * (H + 64) + row * (Q1 > 0 ? Q1 : 1), (row >> 1) & 3, (row >> 2) & 1,
-                                                   half, grp[r], a_addr + dst_off[r], row & 7, chunk0[r]);
+                                                   half, grp[r], a_addr + dst_off[r], swz, chunk0[r]);
             fence_proxy_async_smem();
             __syncwarp();
             signal_a_full(ai, 4);
@@ -590,9 +609,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
         } else if (!BWD) {
             // raw stage = 128 rows x half block = two operand stages (its 64-column halves); groups 0, 1 take the even
             // raw stages, groups 2, 3 the odd ones; a thread owns one row of its group's half
-            const int row = dt, sub = g4 & 1;
+            // (paired rows: operand row dt is row dt >> 1 of the boxes of pair member dt & 1)
+            const int row = p.pair_hb ? (dt >> 1) + (dt & 1) * 64 : dt, sub = g4 & 1;
             const int grp[2] = {2 * sub, 2 * sub + 1};
-            const int prow = p.dual ? dual_row(row) : row;      // (prow & 7 == row & 7: the swizzle phase stays the row's)
+            const int prow = p.dual ? dual_row(row) : dt;      // (prow & 7 == dt & 7)
+            const int hb0 = p.pair_hb && (dt & 1) ? p.pair_hb : 0;
             const uint32_t dst_off[2] = {(uint32_t)(prow * 128), (uint32_t)(prow * 128)};
             const int chunk0[2] = {0, 4};
             for (int ui = g4 >> 1; ui < nu && ok; ui += 2) {
@@ -601,16 +622,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                 if (!ok) break;
                 if (dt == 0 && g4 < 2) trace(2 + 3 * g4, 2 * ui + sub);
                 const uint8_t *rs = smem + kOffRaw + ri * kRawStageBytes;
-                ok = produce(2 * ui + sub, rs, row, (u0 + ui) & 1, grp, dst_off, chunk0);
+                ok = produce(2 * ui + sub, rs, row, dt & 7, (u0 + ui + hb0) & 1, grp, dst_off, chunk0);
                 if (!ok) break;
                 if (lane == 0) mbar_arrive(bar(kBarRawEmpty + raw_bar(ui)));
             }
         } else {
             // raw stage = 64 rows x half block = one operand stage (two 64-column images); group g4 takes the stages
             // ui = g4 (mod 4); a thread owns one row of one image
-            const int row = dt & 63, im = dt >> 6;
+            const int orow = dt & 63, im = dt >> 6;
+            const int row = p.pair_hb ? (orow >> 1) + (orow & 1) * 32 : orow;
+            const int hb0 = p.pair_hb && (orow & 1) ? p.pair_hb : 0;
             const int grp[2] = {2 * im, 2 * im + 1};
-            const uint32_t dst_off[2] = {(uint32_t)(im * 8192 + row * 128), (uint32_t)(im * 8192 + row * 128)};
+            const uint32_t dst_off[2] = {(uint32_t)(im * 8192 + orow * 128), (uint32_t)(im * 8192 + orow * 128)};
             const int chunk0[2] = {0, 4};
             for (int ui = g4; ui < nu && ok; ui += 4) {
                 const int ri = ui % kNumRaw;
@@ -618,7 +641,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                 if (!ok) break;
                 if (dt == 0 && g4 < 2) trace(2 + 3 * g4, ui);
                 const uint8_t *rs = smem + kOffRaw + ri * kRawStageBytes;
-                ok = produce(ui, rs, row, tile & 1, grp, dst_off, chunk0);
+                ok = produce(ui, rs, row, orow & 7, (tile + hb0) & 1, grp, dst_off, chunk0);
                 if (!ok) break;
                 if (lane == 0) mbar_arrive(bar(kBarRawEmpty + raw_bar(ui)));
             }
@@ -1000,8 +1023,29 @@ cudaError_t umma_init_weight_maps(WeightDev *w, const char **err) {
         return cudaSuccess;
     }
     if (w->qtype != kTypeQ4K && w->qtype != kTypeQ6K) return cudaSuccess;
-    if (w->K % 256 != 0 || w->row_bytes == 0) return cudaSuccess;   // flat streams run on the CUDA-core path
     const int H = w->qtype == kTypeQ4K ? 16 : 32;
+    if (w->K % 256 == 128 && w->N % 2 == 0) {
+        // two weight rows are a whole number of super-blocks: maps over [N / 2, 2 K], 64-row boxes (forward: 64 rows of either
+        // member of the pairs per stage) and 32-row boxes (backward), the latter in the *_f maps
+        const uint64_t rb = (uint64_t)(w->K / 128) * dev_block_bytes(w->qtype), rows = (uint64_t)w->N / 2;
+        bool okp = rb % 16 == 0;
+        for (int f = 0; f < 2; f++) {
+            const uint32_t box = f ? 32 : 64;
+            okp = okp && encode_2d(f ? &w->tm_hdr_f : &w->tm_hdr, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, rb, rows, rb, H, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+            okp = okp && encode_2d(f ? &w->tm_q0_f : &w->tm_q0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, rb, rows, rb, 64, box, CU_TENSOR_MAP_SWIZZLE_64B);
+            if (w->qtype == kTypeQ6K)
+                okp = okp && encode_2d(f ? &w->tm_q1_f : &w->tm_q1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, rb, rows, rb, 32, box, CU_TENSOR_MAP_SWIZZLE_32B);
+        }
+        if (!okp) return cudaSuccess;      // the exact kernels take it
+        if (w->qtype == kTypeQ4K) {
+            w->tm_q1 = w->tm_q0;
+            w->tm_q1_f = w->tm_q0_f;
+        }
+        w->pair_hb = w->K / 128;
+        w->tma_ok = true;
+        return cudaSuccess;
+    }
+    if (w->K % 256 != 0 || w->row_bytes == 0) return cudaSuccess;   // other flat streams run on the exact kernels
     bool ok = encode_2d(&w->tm_hdr, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
                         (uint64_t)w->row_bytes, H, 64, CU_TENSOR_MAP_SWIZZLE_NONE);
     ok = ok && encode_2d(&w->tm_hdr_f, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
@@ -1060,7 +1104,8 @@ bool umma_group_ok(const UmmaLaunch *m, int n) {
     if (n < 1 || n > kMaxMembers) return false;
     for (int j = 0; j < n; j++) {
         const WeightDev *w = m[j].w;
-        if (!w || !w->tma_ok || w->qtype != m[0].w->qtype || w->K != m[0].w->K) return false;
+        if (!w || !w->tma_ok || w->qtype != m[0].w->qtype || w->K != m[0].w->K || w->pair_hb != m[0].w->pair_hb) return false;
+        if (w->pair_hb && m[j].rows > 0) return false;
         if (m[j].rank > 64) return false;
         if (w->qtype == kTypeF16 && (!m[j].fp16 || m[j].rank > 0)) return false;      // fp16 rows: fp16 MMA operands, no adapter stage
         if (m[j].row_base < 0 || m[j].row_base + eff_rows(m[j]) > w->N) return false;
@@ -1138,7 +1183,7 @@ int umma_group_splits(const UmmaLaunch *m, int n, int sm_count) {
 bool umma_dual_ok(const UmmaLaunch *m, int sm_count) {
     if (!umma_group_ok(m, 2) || m[0].backward || few_group(m, 2)) return false;
     const WeightDev *a = m[0].w, *b = m[1].w;
-    if (a->qtype == kTypeF16 || a->N != b->N || a->N % 64 != 0 || m[0].rows || m[1].rows) return false;
+    if (a->qtype == kTypeF16 || a->pair_hb || a->N != b->N || a->N % 64 != 0 || m[0].rows || m[1].rows) return false;
     if (m[0].rank > 32 || m[1].rank > 32 || m[0].out_prefilled || m[1].out_prefilled) return false;
     if (m[0].T <= 128) return false;      // the kernel's 256-row activation stages
     // one CTA per 64 features and token chunk, no split-K: worth it where those alone fill the GPU
@@ -1210,10 +1255,11 @@ cudaError_t launch_umma_group(const UmmaLaunch *m, int n, cudaStream_t s, const 
         const UmmaLaunch &L = m[j];
         const WeightDev *w = L.w;
         Member &M = p.m[j];
-        // (64-row boxes: the backward's raw stages, and the dual forward's two half-tiles)
-        M.tm_hdr = (L0.backward || dual) ? w->tm_hdr : w->tm_hdr_f;
-        M.tm_q0 = (L0.backward || dual) ? w->tm_q0 : w->tm_q0_f;
-        M.tm_q1 = (L0.backward || dual) ? w->tm_q1 : w->tm_q1_f;
+        // (64-row boxes: the backward's raw stages, and the dual forward's two half-tiles; paired rows: half of each)
+        const bool small_box = w->pair_hb ? !bwd : (bwd || dual);
+        M.tm_hdr = small_box ? w->tm_hdr : w->tm_hdr_f;
+        M.tm_q0 = small_box ? w->tm_q0 : w->tm_q0_f;
+        M.tm_q1 = small_box ? w->tm_q1 : w->tm_q1_f;
         const int rows = eff_rows(L);
         M.row_base = L.row_base;
         if (bwd || j == 0) {
@@ -1257,6 +1303,7 @@ cudaError_t launch_umma_group(const UmmaLaunch *m, int n, cudaStream_t s, const 
         M.count = count;
         first += count;
     }
+    p.pair_hb = L0.w->pair_hb;
     p.status = L0.status;
     p.trace = (long long *)L0.trace;
     p.T = L0.T;
