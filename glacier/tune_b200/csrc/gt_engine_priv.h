@@ -89,7 +89,8 @@ struct gt_engine {
     double *clip = nullptr;      // device double[2]
     Scratch x16, dy16, dlow, ytmp;
     Scratch ce, ce_host;         // LM-head cross-entropy: logits / probability tiles and per-token state; host staging
-    Scratch attn;                // attention: log-sum-exp rows and the dO.O row sums
+    Scratch attn;                // attention backward: dO.O row sums, 16-bit dO, dk / dv of every query head
+    Scratch attn16;              // 16-bit q, k, v of the attention calls on fp32 tensors
     Scratch low_parts;           // partial sums of X*A of the few-token forward
     Scratch ffn[3];              // gate, up, hidden (forward) / dHidden, dGate, dUp (backward) of the fused FFN calls
     // Host-buffer calls: a ring of staging slots and two copy streams, so that the upload of one call, the kernels
@@ -172,9 +173,12 @@ void drop_step_graphs(gt_engine *e);
 int lm_head_loss_on_device(gt_engine *e, const gt_weight *w, const float *hidden, const int *labels, int T, float *loss_dev, int *valid_dev,
                            float *d_hidden);
 int embedding_on_device(gt_engine *e, const gt_weight *w, const int *tokens, int T, float *out, int *bad_dev);
-// causal GQA attention on device tensors (gt_attention.cu); lse: [heads_q, T] fp32 kept for the backward
-int attention_forward_on_device(gt_engine *e, const float *q, const float *k, const float *v, float *out, float *lse, int T, int heads_q,
-                                int heads_kv, int head_dim);
-int attention_backward_on_device(gt_engine *e, const float *d_out, const float *q, const float *k, const float *v, const float *out,
-                                 const float *lse, float *dq, float *dk, float *dv, int T, int heads_q, int heads_kv, int head_dim);
+// causal GQA attention on device tensors (gt_attention.cu); lse: [heads_q, T] fp32 kept for the backward.  The 16-bit operands
+// (q16 scaled for base-2 scores, q16 and k16 rotated when rope_freq_base > 0) are what both directions read.
+int attention_operands_on_device(gt_engine *e, const float *q, const float *k, const float *v, void *q16, void *k16, void *v16, int T, int heads_q,
+                                 int heads_kv, float rope_freq_base);
+int attention_forward16_on_device(gt_engine *e, const void *q16, const void *k16, const void *v16, float *out, float *lse, int T, int heads_q,
+                                  int heads_kv, int head_dim);
+int attention_backward16_on_device(gt_engine *e, const float *d_out, const void *q16, const void *k16, const void *v16, const float *out, const float *lse,
+                                   float *dq, float *dk, float *dv, int T, int heads_q, int heads_kv, int head_dim);
 }  // namespace gt

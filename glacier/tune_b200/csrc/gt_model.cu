@@ -27,7 +27,8 @@ namespace {
 enum { kQ = 0, kK, kV, kO, kGate, kUp, kDown, kProj };
 
 struct BlockState {      // what a block's backward needs from its forward
-    float *n1, *q, *k, *v, *attn, *lse, *x1, *n2, *gate, *up, *hidden;
+    float *n1, *attn, *lse, *x1, *n2, *gate, *up, *hidden;
+    void *q16, *k16, *v16;      // the attention's operands: q, k rotated (q scaled), v, rounded to 16 bits
 };
 struct LayerDev {
     const gt_weight *w[kProj] = {};
@@ -48,6 +49,7 @@ struct gt_model {
     std::vector<float *> x;            // x[l] = input of block l, x[L] = output of the last block; [T, hidden] each
     std::vector<BlockState> st;        // one set (checkpointing) or one per block
     float *tmp_h = nullptr;            // projection output before the residual add
+    float *q = nullptr, *k = nullptr, *v = nullptr;      // q, k, v projections of the block at hand
     float *fnorm = nullptr, *dfnorm = nullptr, *dx_a = nullptr, *dx_b = nullptr, *dn = nullptr, *dx1 = nullptr;
     float *dattn = nullptr, *dq = nullptr, *dk = nullptr, *dv = nullptr;
     int *tokens = nullptr, *labels = nullptr, *valid = nullptr, *bad = nullptr;
@@ -105,11 +107,12 @@ int block_forward(gt_model *m, int l, const float *x_in, float *x_out, BlockStat
     const LayerDev &L = m->layers[l];
     const int H = c.hidden;
     if (!n1_ready) GT_LAUNCH(e, launch_rmsnorm_fwd(x_in, L.norm1, s.n1, T, H, c.rms_eps, e->stream));
-    float *qkv[3] = {s.q, s.k, s.v};
+    float *qkv[3] = {m->q, m->k, m->v};
     int rc = forward_group_device(e, 3, L.w + kQ, L.ad + kQ, s.n1, qkv, T, 0);
     if (rc != GT_OK) return rc;
-    GT_LAUNCH(e, launch_rope(s.q, s.k, T, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_theta, 1.0f, c.head_dim, 0, e->stream));
-    rc = attention_forward_on_device(e, s.q, s.k, s.v, s.attn, s.lse, T, c.n_heads, c.n_kv_heads, c.head_dim);
+    // RoPE on q and k, and the 16-bit operands of the attention and of its backward, in one pass
+    rc = attention_operands_on_device(e, m->q, m->k, m->v, s.q16, s.k16, s.v16, T, c.n_heads, c.n_kv_heads, c.rope_theta);
+    if (rc == GT_OK) rc = attention_forward16_on_device(e, s.q16, s.k16, s.v16, s.attn, s.lse, T, c.n_heads, c.n_kv_heads, c.head_dim);
     if (rc != GT_OK) return rc;
     float *o = m->tmp_h;
     rc = forward_group_device(e, 1, L.w + kO, L.ad + kO, s.attn, &o, T, 0);
@@ -147,7 +150,7 @@ int block_backward(gt_model *m, int l, const float *d_out, const float *x_in, co
     const float *dy_o = m->dx1;
     rc = backward_group_device(e, 1, L.w + kO, L.ad + kO, &dy_o, s.attn, m->dattn, T, flags);
     if (rc != GT_OK) return rc;
-    rc = attention_backward_on_device(e, m->dattn, s.q, s.k, s.v, s.attn, s.lse, m->dq, m->dk, m->dv, T, c.n_heads, c.n_kv_heads, c.head_dim);
+    rc = attention_backward16_on_device(e, m->dattn, s.q16, s.k16, s.v16, s.attn, s.lse, m->dq, m->dk, m->dv, T, c.n_heads, c.n_kv_heads, c.head_dim);
     if (rc != GT_OK) return rc;
     GT_LAUNCH(e, launch_rope(m->dq, m->dk, T, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_theta, 1.0f, c.head_dim, 1, e->stream));
     const float *dqkv[3] = {m->dq, m->dk, m->dv};
@@ -234,9 +237,10 @@ int gt_model_create(gt_engine *e, const gt_model_config *cfg, gt_model **out) {
     const size_t T = c.max_tokens, H = c.hidden, F = c.ffn, QD = (size_t)c.n_heads * c.head_dim, KD = (size_t)c.n_kv_heads * c.head_dim;
     const int n_state = c.checkpoint ? 1 : c.n_layers;
     const size_t bh = a256(T * H * 4), bf = a256(T * F * 4), bq = a256(T * QD * 4), bk = a256(T * KD * 4), bl = a256((size_t)c.n_heads * T * 4);
-    const size_t state_bytes = 3 * bh + 2 * bq + 2 * bk + bl + 3 * bf;       // n1, x1, n2 | q, attn | k, v | lse | gate, up, hidden
+    const size_t bq16 = a256(T * QD * 2), bk16 = a256(T * KD * 2);
+    const size_t state_bytes = 3 * bh + bq + bq16 + 2 * bk16 + bl + 3 * bf;       // n1, x1, n2 | attn | q16 | k16, v16 | lse | gate, up, hidden
     size_t total = (size_t)(c.n_layers + 1) * bh + (size_t)n_state * state_bytes + 7 * bh /* tmp, fnorm, dfnorm, dx_a, dx_b, dn, dx1 */ +
-                   2 * bq /* dattn, dq */ + 2 * bk + 2 * a256(T * 4) + 1024;
+                   3 * bq /* q, dattn, dq */ + 4 * bk /* k, v, dk, dv */ + 2 * a256(T * 4) + 1024;
     cudaError_t ce = cudaMalloc((void **)&m->arena, total);
     if (ce != cudaSuccess) {
         delete m;
@@ -254,14 +258,14 @@ int gt_model_create(gt_engine *e, const gt_model_config *cfg, gt_model **out) {
     m->st.resize(n_state);
     for (BlockState &s : m->st) {
         s.n1 = take(bh); s.x1 = take(bh); s.n2 = take(bh);
-        s.q = take(bq); s.attn = take(bq);
-        s.k = take(bk); s.v = take(bk);
+        s.attn = take(bq);
+        s.q16 = take(bq16); s.k16 = take(bk16); s.v16 = take(bk16);
         s.lse = take(bl);
         s.gate = take(bf); s.up = take(bf); s.hidden = take(bf);
     }
     m->tmp_h = take(bh); m->fnorm = take(bh); m->dfnorm = take(bh); m->dx_a = take(bh); m->dx_b = take(bh); m->dn = take(bh); m->dx1 = take(bh);
-    m->dattn = take(bq); m->dq = take(bq);
-    m->dk = take(bk); m->dv = take(bk);
+    m->q = take(bq); m->dattn = take(bq); m->dq = take(bq);
+    m->k = take(bk); m->v = take(bk); m->dk = take(bk); m->dv = take(bk);
     m->tokens = (int *)take(a256(T * 4));
     m->labels = (int *)take(a256(T * 4));
     m->loss = take(256);
