@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(32 * Shape<T1>::WARPS, 1) k_decode(const __gri
             for (int bl = 0; bl < nblk; bl++) {
                 const int b = cs.c * kQ4Chunk + bl;
                 {   // lane (row = lane & 15, half = lane >> 4) turns four (sc, m) pairs of its row into (a, c = 128 a + b)
-                    const uint4 h = lds128(stage + (lane & 15) * kQ4Row + bl * kQ4KBlockBytes);
+                    const uint4 h = lds128(stage + (lane & 15) * kQ4Row + bl * kQ4KBlockBytes + kQ4KHdr);
                     const float d = half_bits_to_f32(h.x & 0xFFFFu), dmin = half_bits_to_f32(h.x >> 16);
                     const bool hi = lane >= 16;
                     const uint32_t sc4 = hi ? ((h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u)) : (h.y & 0x3F3F3F3Fu);
@@ -450,11 +450,12 @@ __global__ void __launch_bounds__(32 * Shape<T1>::WARPS, 1) k_decode(const __gri
                     }
                     __syncwarp();
                 }
-                const uint32_t qa = stage + g * kQ4Row + bl * kQ4KBlockBytes + 16 + t4 * 8, qb = qa + 8 * kQ4Row;
+                const uint32_t qa = stage + g * kQ4Row + bl * kQ4KBlockBytes + t4 * 8, qb = qa + 8 * kQ4Row;
                 const uint32_t xb = xg + b * x_step + t4 * (T1 ? 8 : 16);
 #pragma unroll
                 for (int j = 0; j < 4; j++) {      // sub-blocks 2j (low nibbles) and 2j + 1 (high)
-                    const uint2 ca = lds64(qa + j * 32), cb = lds64(qb + j * 32);
+                    const uint32_t qo = j * 32 + (j >> 1) * 16;      // (the header sits between the halves)
+                    const uint2 ca = lds64(qa + qo), cb = lds64(qb + qo);
                     // (a, c) of the two sub-blocks for rows g and g + 8; one token: a alone
                     float4 sa, sc;
                     if (T1) {
@@ -499,9 +500,9 @@ __global__ void __launch_bounds__(32 * Shape<T1>::WARPS, 1) k_decode(const __gri
         } else {
             const int b = cs.c;
             {   // lane (row, step = lane >> 4): eight scales of its row, stored in (step, half, quad) order
-                const uint32_t hdr = stage + (lane & 15) * kQ6Row;
-                const uint2 s8 = lds64(hdr + (lane >> 4) * 8);
-                const float d = half_bits_to_f32(lds32(hdr + 16) & 0xFFFFu);
+                const uint4 h = lds128(stage + (lane & 15) * kQ6Row + (lane >> 4) * kQ6KHalf);
+                const uint2 s8 = make_uint2(h.x, h.y);
+                const float d = half_bits_to_f32(h.z & 0xFFFFu);
                 float v[8];      // byte index = quad * 2 + half
 #pragma unroll
                 for (int q = 0; q < 8; q++) v[q] = d * (float)(int8_t)(((q < 4 ? s8.x : s8.y) >> (8 * (q & 3))) & 255u);
@@ -525,7 +526,7 @@ __global__ void __launch_bounds__(32 * Shape<T1>::WARPS, 1) k_decode(const __gri
 #pragma unroll
             for (int sh = 0; sh < 4; sh++) {      // (step, half): four sub-blocks of 16, quads 0..3
                 const int step = sh >> 1, hf = sh & 1;
-                const uint32_t lo = 32 + step * 64 + hf * 16 + t4 * 4, ho = 160 + step * 32 + hf * 16 + t4 * 4;
+                const uint32_t lo = 16 + step * kQ6KHalf + hf * 16 + t4 * 4, ho = 80 + step * kQ6KHalf + hf * 16 + t4 * 4;
                 const uint32_t la[2] = {lds32(ra + lo), lds32(ra + lo + 32)}, lb[2] = {lds32(rb + lo), lds32(rb + lo + 32)};
                 const uint32_t ha = lds32(ra + ho), hb = lds32(rb + ho);
                 const float4 fa = lds128f(scr + (g * 16 + sh * 4) * 4), fb = lds128f(scr + ((g + 8) * 16 + sh * 4) * 4);

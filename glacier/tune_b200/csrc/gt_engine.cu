@@ -1130,6 +1130,7 @@ int gt_weight_upload(gt_engine *e, int ggml_type, const void *host_bytes, int64_
         d.nbytes = nbytes;
         ce = cudaMalloc((void **)&d.data, d.nbytes);
         if (ce == cudaSuccess) ce = cudaMemcpyAsync(d.data, host_bytes, nbytes, cudaMemcpyHostToDevice, e->stream);
+        if (ce == cudaSuccess && ggml_type == GT_TYPE_Q4_K) ce = launch_q4k_repack(d.data, nelem / 256, e->stream);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     }
     if (ce == cudaSuccess && bias) {

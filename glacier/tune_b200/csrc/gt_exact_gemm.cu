@@ -84,8 +84,8 @@ struct Run8<kTypeQ4K> {
     __device__ __forceinline__ void load(const uint8_t *w, int64_t e, int) {
         const uint8_t *b = w + (e >> 8) * kQ4KBlockBytes;
         const int c = (int)(e & 255);
-        h = __ldg(reinterpret_cast<const uint4 *>(b));
-        q = __ldg(reinterpret_cast<const uint2 *>(b + 16 + (c >> 6) * 32 + (c & 31)));
+        h = __ldg(reinterpret_cast<const uint4 *>(b + kQ4KHdr));
+        q = __ldg(reinterpret_cast<const uint2 *>(b + (c >> 7) * 80 + ((c >> 6) & 1) * 32 + (c & 31)));
     }
     __device__ __forceinline__ void decode(int64_t e, float (&v)[8]) const {
         const int ib = (int)(e & 255) >> 5;
@@ -103,12 +103,12 @@ struct Run8<kTypeQ6K> {
     uint16_t d;
     int8_t sc;
     __device__ __forceinline__ void load(const uint8_t *w, int64_t e, int) {
-        const uint8_t *b = w + (e >> 8) * kQ6KDevBlockBytes;
-        const int c = (int)(e & 255), step = c >> 7, quad = (c & 127) >> 5, ln = c & 31;
-        l = __ldg(reinterpret_cast<const uint2 *>(b + 32 + step * 64 + (quad & 1) * 32 + ln));
-        hb = __ldg(reinterpret_cast<const uint2 *>(b + 160 + step * 32 + ln));
-        d = __ldg(reinterpret_cast<const uint16_t *>(b + 16));
-        sc = __ldg(reinterpret_cast<const int8_t *>(b) + step * 8 + (ln >> 4) + quad * 2);
+        const uint8_t *b = w + (e >> 7) * kQ6KHalf;
+        const int quad = (int)(e & 127) >> 5, ln = (int)(e & 31);
+        l = __ldg(reinterpret_cast<const uint2 *>(b + 16 + (quad & 1) * 32 + ln));
+        hb = __ldg(reinterpret_cast<const uint2 *>(b + 80 + ln));
+        d = __ldg(reinterpret_cast<const uint16_t *>(b + 8));
+        sc = __ldg(reinterpret_cast<const int8_t *>(b) + (ln >> 4) + quad * 2);
     }
     __device__ __forceinline__ void decode(int64_t e, float (&v)[8]) const {
         const int quad = ((int)(e & 127)) >> 5, ls = (quad >> 1) * 4, hs = quad * 2;

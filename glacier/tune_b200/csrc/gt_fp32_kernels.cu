@@ -7,7 +7,7 @@
 namespace gt {
 
 // ------------------------------------------------------------------------------------------------
-// Q6_K upload re-layout: GGUF 210-byte block -> 224-byte device block (see gt_quant.cuh).
+// Upload re-layouts, a warp per super-block (see gt_quant.cuh): Q6_K 210-byte GGUF block -> 224-byte device block; Q4_K in place.
 // ------------------------------------------------------------------------------------------------
 __global__ void k_q6k_repack(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int64_t nblocks) {
     const int64_t b = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
@@ -15,15 +15,32 @@ __global__ void k_q6k_repack(const uint8_t *__restrict__ src, uint8_t *__restric
     const int lane = threadIdx.x & 31;
     const uint8_t *s = src + b * kQ6KGgufBlockBytes;
     uint8_t *d = dst + b * kQ6KDevBlockBytes;
-    for (int i = lane; i < 224; i += 32) {
+    for (int i = lane; i < kQ6KDevBlockBytes; i += 32) {
+        const int half = i / kQ6KHalf, k = i % kQ6KHalf;
         uint8_t v = 0;
-        if (i < 16) v = s[192 + i];            // scales
-        else if (i < 18) v = s[208 + (i - 16)];  // d
-        else if (i < 32) v = 0;
-        else if (i < 160) v = s[i - 32];       // ql
-        else v = s[128 + (i - 160)];           // qh
+        if (k < 8) v = s[192 + 8 * half + k];              // scales
+        else if (k < 10) v = s[208 + (k - 8)];             // d
+        else if (k < 16) v = 0;
+        else if (k < 80) v = s[64 * half + (k - 16)];      // ql
+        else v = s[128 + 32 * half + (k - 80)];            // qh
         d[i] = v;
     }
+}
+__global__ void k_q4k_repack(uint8_t *data, int64_t nblocks) {
+    const int64_t b = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    if (b >= nblocks) return;
+    const int lane = threadIdx.x & 31;
+    uint32_t *w = reinterpret_cast<uint32_t *>(data + b * kQ4KBlockBytes);      // 4 header words, 32 words of quants
+    const uint32_t q = w[4 + lane], h = lane < 4 ? w[lane] : 0u;
+    __syncwarp();
+    w[lane < 16 ? lane : lane + 4] = q;
+    if (lane < 4) w[kQ4KHdr / 4 + lane] = h;
+}
+cudaError_t launch_q4k_repack(uint8_t *blocks, int64_t nblocks, cudaStream_t s) {
+    if (nblocks <= 0) return cudaSuccess;
+    const int wpb = 8;
+    k_q4k_repack<<<(unsigned)((nblocks + wpb - 1) / wpb), wpb * 32, 0, s>>>(blocks, nblocks);
+    return cudaGetLastError();
 }
 cudaError_t launch_q6k_repack(const uint8_t *gguf_blocks, uint8_t *dev_blocks, int64_t nblocks, cudaStream_t s) {
     if (nblocks <= 0) return cudaSuccess;

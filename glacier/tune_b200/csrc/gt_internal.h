@@ -32,19 +32,20 @@ cudaError_t per_device_once(PerDeviceOnce &st, F &&fn) {
 struct WeightDev {
     int qtype = 0;
     int N = 0, K = 0;             // [out_features, in_features]
-    uint8_t *data = nullptr;      // device blocks (Q4_K: GGUF bytes; Q6_K: 224-byte device blocks; F32: floats)
+    uint8_t *data = nullptr;      // device blocks (K-quants: the layouts of gt_quant.cuh; F32: floats)
     int64_t nbytes = 0;
     int64_t row_bytes = 0;        // K/256 * block bytes when K % 256 == 0, else 0 (flat super-block stream)
     float *bias = nullptr;        // [N] or null
     bool tma_ok = false;          // tensor maps built: rows of whole super-blocks, or pairs of rows
     int pair_hb = 0;              // maps over pairs of rows (in_features % 256 == 128): half super-blocks per row, else 0
-    CUtensorMap tm_hdr, tm_q0, tm_q1;   // 2-D byte maps over [N, row_bytes], boxes of 64 rows (backward raw stages)
-    CUtensorMap tm_hdr_f, tm_q0_f, tm_q1_f;   // the same with boxes of 128 rows (forward raw stages: half as many copies)
+    CUtensorMap tm16_f, tm16_b;         // F16: 64-column boxes of 128 rows (forward) / 64 rows (backward)
     CUtensorMap tm_rows;                // 32-bit words over [N, row_bytes / 4], boxes of 16 rows x two Q4_K blocks / one Q6_K block
-    CUtensorMap tm_blk_f, tm_blk_b;     // whole super-blocks: boxes of one block x 256 rows / x 64 rows (few-token kernel)
+    CUtensorMap tm_blk_f, tm_blk;       // K-quants: boxes of one super-block x 256 rows (few-token kernel) / x 64 rows
+    CUtensorMap tm_half, tm_half_p;     // boxes of half a super-block x 64 rows (or pairs of rows) / x 32 pairs
 };
 
 // ---- CUDA-core kernels (gt_fp32_kernels.cu) -------------------------------------------------------------
+cudaError_t launch_q4k_repack(uint8_t *blocks, int64_t nblocks, cudaStream_t s);      // in place
 cudaError_t launch_q6k_repack(const uint8_t *gguf_blocks, uint8_t *dev_blocks, int64_t nblocks, cudaStream_t s);
 cudaError_t launch_dequant_rows(int qt, const uint8_t *w, int K, int64_t row0, int64_t nrows, float *out, cudaStream_t s);
 // ---- fp32-accurate GEMMs on exact weights, any type and shape (gt_exact_gemm.cu)

@@ -1,10 +1,12 @@
 // GGUF K-quant block formats as they sit in HBM, and their decoders.
 //
-// Q4_K keeps the GGUF layout (144 B, 16-byte aligned fields):
-//     [0,2) half d   [2,4) half dmin   [4,16) u8 scales[12]   [16,144) u8 qs[128]
-// Q6_K is re-laid out at upload so that every field starts on a 16-byte boundary (TMA needs it; the GGUF
-// block is 210 B).  Device block, 224 B:
-//     [0,16) i8 scales[16]   [16,18) half d   [18,32) pad   [32,160) u8 ql[128]   [160,224) u8 qh[64]
+// Both K-quants are re-laid out at upload, so that whatever a kernel needs of one half of a super-block (128 weights) is ONE run of
+// bytes that starts and ends on a 16-byte boundary: a tiled TMA copy of it is one request per weight row, and the requests are what
+// those copies cost (4 to 5 clocks each).  The odd multiples of 16 bytes also keep row-per-thread reads of a stage free of bank conflicts.
+// Q4_K device block, 144 B - the halves share the header between them: half h is [64 h, 64 h + 80):
+//     [0,64) u8 qs[0..63]   [64,66) half d   [66,68) half dmin   [68,80) u8 scales[12]   [80,144) u8 qs[64..127]
+// Q6_K device block, 224 B (GGUF: 210 B) - half h is [112 h, 112 h + 112), d is stored in both:
+//     [0,8) i8 scales[8 h..]   [8,10) half d   [10,16) pad   [16,80) u8 ql[64 h..]   [80,112) u8 qh[32 h..]
 // Decoded values are identical to the reference decode
 // (src/Glacier.Tune/Gpu/Kernels/tune_bwd.cu:43-51,209-211,234-240,279-289,311-315): every product is exact in
 // fp32 and Q4_K's final subtraction rounds once, fused or not.
@@ -29,6 +31,12 @@ constexpr int kQ6KGgufBlockBytes = 210;
 constexpr int kQ6KDevBlockBytes = 224;
 constexpr int kQ40BlockBytes = 18;
 constexpr int kQ80BlockBytes = 34;
+
+constexpr int kQ4KHdr = 64;            // header of a Q4_K device block; quants of half h at 80 h
+constexpr int kQ6KHalf = 112;          // bytes of half a Q6_K device block
+// half a super-block: its bytes, and the distance between the starts of the two
+__host__ __device__ constexpr int dev_half_bytes(int qt) { return qt == kTypeQ4K ? 80 : (qt == kTypeQ6K ? kQ6KHalf : 0); }
+__host__ __device__ constexpr int dev_half_step(int qt) { return qt == kTypeQ4K ? kQ4KHdr : (qt == kTypeQ6K ? kQ6KHalf : 0); }
 
 __host__ __device__ constexpr int dev_block_bytes(int qt) {
     return qt == kTypeQ4K ? kQ4KBlockBytes : (qt == kTypeQ6K ? kQ6KDevBlockBytes : 0);
@@ -63,23 +71,24 @@ __device__ __forceinline__ void q4k_scale_min_w(int j, uint32_t w0, uint32_t w1,
 
 // Exact fp32 value of element c (0..255) of one block.
 __device__ __forceinline__ float q4k_decode_elem(const uint8_t *blk, int c) {
-    const float d = half_bits_to_f32(*(const uint16_t *)blk);
-    const float dmin = half_bits_to_f32(*(const uint16_t *)(blk + 2));
+    const float d = half_bits_to_f32(*(const uint16_t *)(blk + kQ4KHdr));
+    const float dmin = half_bits_to_f32(*(const uint16_t *)(blk + kQ4KHdr + 2));
     const int ib = c >> 5;
     int sc, m;
-    q4k_scale_min(ib, blk + 4, sc, m);
-    const int q = (blk[16 + (ib >> 1) * 32 + (c & 31)] >> ((ib & 1) * 4)) & 0x0F;
+    q4k_scale_min(ib, blk + kQ4KHdr + 4, sc, m);
+    const int q = (blk[(c >> 7) * 80 + ((ib >> 1) & 1) * 32 + (c & 31)] >> ((ib & 1) * 4)) & 0x0F;
     const float d_sub = d * (float)sc;
     const float m_sub = dmin * (float)m;
     return d_sub * (float)q - m_sub;
 }
 __device__ __forceinline__ float q6k_dev_decode_elem(const uint8_t *blk, int c) {
     const int step = c >> 7, rem = c & 127, quad = rem >> 5, lane = rem & 31;
-    const int ql = blk[32 + step * 64 + (quad & 1) * 32 + lane];
-    const int qh = blk[160 + step * 32 + lane];
+    blk += step * kQ6KHalf;
+    const int ql = blk[16 + (quad & 1) * 32 + lane];
+    const int qh = blk[80 + lane];
     const int q = (int)(((ql >> (quad >= 2 ? 4 : 0)) & 0x0F) | (((qh >> (quad * 2)) & 0x03) << 4)) - 32;
-    const float d = half_bits_to_f32(*(const uint16_t *)(blk + 16));
-    const int sc = (int)(int8_t)blk[step * 8 + (lane >> 4) + quad * 2];
+    const float d = half_bits_to_f32(*(const uint16_t *)(blk + 8));
+    const int sc = (int)(int8_t)blk[(lane >> 4) + quad * 2];
     return d * (float)sc * (float)q;
 }
 // Q4_0 (src/Glacier.Tune/Gpu/Kernels/tune_bwd.cu:23-26,151-163): weight i of a block = d * (nibble - 8), nibble = low half
@@ -113,41 +122,36 @@ __device__ __forceinline__ float decode_flat(const uint8_t *w, int64_t e) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// 32-element group decoders used by the tensor-core kernels.  A "half block" is 128 consecutive weights of
-// one super-block (half = 0/1); it is staged in shared memory as three row-major regions
-//     hdr  : kHdrBytes per row   (Q4_K: d, dmin, scales[12];  Q6_K: scales[16], d, pad)
-//     q0   : 64 B per row        (Q4_K: qs[64*half ..];       Q6_K: ql[64*half ..])
-//     q1   : 32 B per row        (Q6_K only: qh[32*half ..])
-// Group grp (0..3) is weights [32*grp, 32*grp+32) of the half block.
+// Decoders of the tensor-core kernels.  A thread takes 64 consecutive weights of one super-block - quarter `pair` (0, 1) of
+// half `half` (0, 1), whose bytes start at hp - into registers (Raw64::load) and writes them as two 32-weight groups
+// (dequant32_to_swizzled_row).
 // ------------------------------------------------------------------------------------------------
 template <int QT>
-struct QuantStage;
+struct Raw64;
 template <>
-struct QuantStage<kTypeQ4K> {
-    static constexpr int kHdrBytes = 16, kQ0Bytes = 64, kQ1Bytes = 0;
-    static constexpr int kBlockBytes = kQ4KBlockBytes;
-    __host__ __device__ static constexpr int hdr_x(int /*half*/) { return 0; }
-    __host__ __device__ static constexpr int q0_x(int half) { return 16 + 64 * half; }
-    __host__ __device__ static constexpr int q1_x(int /*half*/) { return 0; }
+struct Raw64<kTypeQ4K> {
+    uint4 h, qa, qb;      // d, dmin, scales[12]; 32 bytes of quants: low nibbles = the first 32 weights, high nibbles = the next
+    __device__ __forceinline__ void load(const uint8_t *hp, int half, int pair) {
+        h = *reinterpret_cast<const uint4 *>(hp + (half ? 0 : kQ4KHdr));
+        const uint4 *q = reinterpret_cast<const uint4 *>(hp + 16 * half + 32 * pair);
+        qa = q[0];
+        qb = q[1];
+    }
 };
 template <>
-struct QuantStage<kTypeQ6K> {
-    static constexpr int kHdrBytes = 32, kQ0Bytes = 64, kQ1Bytes = 32;
-    static constexpr int kBlockBytes = kQ6KDevBlockBytes;
-    __host__ __device__ static constexpr int hdr_x(int /*half*/) { return 0; }
-    __host__ __device__ static constexpr int q0_x(int half) { return 32 + 64 * half; }
-    __host__ __device__ static constexpr int q1_x(int half) { return 160 + 32 * half; }
-};
-
-// fp16 rows need no staging area and no decoder: TMA writes them straight into the operand stage.  The constants only
-// keep the kernel's (unused) packed-block ring well-formed.
-template <>
-struct QuantStage<kTypeF16> {
-    static constexpr int kHdrBytes = 16, kQ0Bytes = 64, kQ1Bytes = 0;
-    static constexpr int kBlockBytes = 512;
-    __host__ __device__ static constexpr int hdr_x(int) { return 0; }
-    __host__ __device__ static constexpr int q0_x(int) { return 0; }
-    __host__ __device__ static constexpr int q1_x(int) { return 0; }
+struct Raw64<kTypeQ6K> {
+    uint32_t sc, d;       // four sub-scales; d in the low half
+    uint4 l[4], ha, hb;   // 64 bytes of ql (the pair picks a nibble), 32 bytes of qh
+    __device__ __forceinline__ void load(const uint8_t *hp, int, int pair) {
+        sc = *reinterpret_cast<const uint32_t *>(hp + 4 * pair);
+        d = *reinterpret_cast<const uint16_t *>(hp + 8);
+        const uint4 *q = reinterpret_cast<const uint4 *>(hp + 16);
+#pragma unroll
+        for (int i = 0; i < 4; i++) l[i] = q[i];
+        const uint4 *hq = reinterpret_cast<const uint4 *>(hp + 80);
+        ha = hq[0];
+        hb = hq[1];
+    }
 };
 
 template <typename T16>
@@ -195,13 +199,8 @@ __device__ __forceinline__ uint32_t bf16x2_splat(float v) {
     return *reinterpret_cast<uint32_t *>(&t);
 }
 
-// Decode group `grp` of half block `half` of one weight row and write its 32 values as four 16-byte chunks of
-// a 128-byte-swizzled operand row: chunk (chunk0 + i) lands at dst_row + (((chunk0 + i) ^ swz) << 4),
-// swz = (row index within the 1024-byte atom) & 7.
-//
-// The raw q0 / q1 regions were written by TMA with 64-byte / 32-byte swizzle (conflict-free reads when the
-// lanes of a warp walk consecutive rows): 16-byte chunk c of a q0 row sits at (c ^ rsw0) << 4, of a q1 row at
-// (c ^ rsw1) << 4, with rsw0 = (row >> 1) & 3 and rsw1 = (row >> 2) & 1.
+// Write group e (0, 1) of a thread's 64 weights as four 16-byte chunks of a 128-byte-swizzled operand row: chunk (chunk0 + i)
+// lands at dst_row + (((chunk0 + i) ^ swz) << 4), swz = (row index within the 1024-byte atom) & 7.
 //
 // T16 = __half : every weight is evaluated exactly in fp32 (the reference formula) and rounded once.
 // T16 = bf16   : packed bf16x2 arithmetic.  A 4-bit quant q is placed in a bf16 mantissa as v = 1 + q/16
@@ -209,23 +208,17 @@ __device__ __forceinline__ uint32_t bf16x2_splat(float v) {
 //                v = 1 + q/64, then w = (64a) * (v - 1.5) with an exact subtraction.  The per-sub-block
 //                constants are rounded to bf16, which adds an error of the size of the bf16 rounding of w itself.
 template <int QT, typename T16>
-__device__ __forceinline__ void dequant32_to_swizzled_row(const uint8_t *hdr_row, const uint8_t *q0_row,
-                                                          const uint8_t *q1_row, int rsw0, int rsw1, int half, int grp,
-                                                          uint32_t dst_row, int swz, int chunk0) {
+__device__ __forceinline__ void dequant32_to_swizzled_row(const Raw64<QT> &raw, int half, int pair, int e, uint32_t dst_row, int swz, int chunk0) {
     constexpr bool kFast = std::is_same<T16, __nv_bfloat16>::value;
-    if constexpr (QT == kTypeF16) {
-        // never called: fp16 tiles are written by TMA
-    } else if constexpr (QT == kTypeQ4K) {
-        const uint4 h = *reinterpret_cast<const uint4 *>(hdr_row);
-        const float d = half_bits_to_f32(h.x & 0xFFFFu);
-        const float dmin = half_bits_to_f32(h.x >> 16);
+    const int grp = 2 * pair + e;
+    if constexpr (QT == kTypeQ4K) {
+        const float d = half_bits_to_f32(raw.h.x & 0xFFFFu);
+        const float dmin = half_bits_to_f32(raw.h.x >> 16);
         int sc, m;
-        q4k_scale_min_w(4 * half + grp, h.y, h.z, h.w, sc, m);
+        q4k_scale_min_w(4 * half + grp, raw.h.y, raw.h.z, raw.h.w, sc, m);
         const float a = d * (float)sc;
         const float b = dmin * (float)m;
-        const int c0 = (grp >> 1) * 2;
-        const uint4 qa = *reinterpret_cast<const uint4 *>(q0_row + ((c0 ^ rsw0) << 4));
-        const uint4 qb = *reinterpret_cast<const uint4 *>(q0_row + (((c0 + 1) ^ rsw0) << 4));
+        const uint4 qa = raw.qa, qb = raw.qb;
         const uint32_t w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
         if constexpr (kFast) {
             const uint32_t a16 = bf16x2_splat(16.f * a);
@@ -262,17 +255,12 @@ __device__ __forceinline__ void dequant32_to_swizzled_row(const uint8_t *hdr_row
             }
         }
     } else {
-        const uint32_t scw = *reinterpret_cast<const uint32_t *>(hdr_row + 8 * half + (grp & 2) * 2);
-        // bytes of scw: scales[8*half + 4*(grp>>1) + 0..3]; this group uses 2*(grp&1) and 2*(grp&1)+1
-        const int s0 = (int)(int8_t)((scw >> (16 * (grp & 1))) & 0xFF);
-        const int s1 = (int)(int8_t)((scw >> (16 * (grp & 1) + 8)) & 0xFF);
-        const float d = half_bits_to_f32(*reinterpret_cast<const uint16_t *>(hdr_row + 16));
+        // bytes of raw.sc: this group uses 2 e and 2 e + 1
+        const int s0 = (int)(int8_t)((raw.sc >> (16 * e)) & 0xFF);
+        const int s1 = (int)(int8_t)((raw.sc >> (16 * e + 8)) & 0xFF);
+        const float d = half_bits_to_f32(raw.d);
         const float a0 = d * (float)s0, a1 = d * (float)s1;
-        const int c0 = (grp & 1) * 2;
-        const uint4 la = *reinterpret_cast<const uint4 *>(q0_row + ((c0 ^ rsw0) << 4));
-        const uint4 lb = *reinterpret_cast<const uint4 *>(q0_row + (((c0 + 1) ^ rsw0) << 4));
-        const uint4 ha = *reinterpret_cast<const uint4 *>(q1_row + ((0 ^ rsw1) << 4));
-        const uint4 hb = *reinterpret_cast<const uint4 *>(q1_row + ((1 ^ rsw1) << 4));
+        const uint4 la = raw.l[2 * e], lb = raw.l[2 * e + 1], ha = raw.ha, hb = raw.hb;
         const uint32_t lw[8] = {la.x, la.y, la.z, la.w, lb.x, lb.y, lb.z, lb.w};
         const uint32_t hw[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
         if constexpr (kFast) {

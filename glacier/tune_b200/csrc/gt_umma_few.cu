@@ -99,8 +99,7 @@ enum { kFewProducer = 600, kFewMma = 700, kFewDequant = 800, kFewEpilogue = 900 
 // slots a dequant group owns two pairs of them: it fills one pair while the MMAs of the other are still queued.
 template <int QT, typename T16, bool BWD, int XROWS>
 __global__ void __launch_bounds__(kThreadsF, 1) k_umma_few(const __grid_constant__ FewParams p) {
-    using QS = QuantStage<QT>;
-    constexpr int BB = QS::kBlockBytes;             // bytes of a super-block = row pitch of a raw stage
+    constexpr int BB = dev_block_bytes(QT);             // bytes of a super-block = row pitch of a raw stage
     constexpr int kRows = BWD ? 64 : kTileN;        // weight rows of a raw stage
     constexpr int kRawStageBytes = (kRows * BB + 1023) & ~1023;
     constexpr int kPerRaw = BWD ? 2 : 8;            // weight stages per raw stage
@@ -279,10 +278,11 @@ __global__ void __launch_bounds__(kThreadsF, 1) k_umma_few(const __grid_constant
                     ok = wait_slot(n) && wait_slot(n + 1);
                     if (!ok) break;
                     if (dt == 0 && g2 == 0) trace(3, 2 * ui + pp);
+                    Raw64<QT> raw;
+                    raw.load(rr + half * dev_half_step(QT), half, q & 1);
 #pragma unroll
                     for (int e = 0; e < 2; e++)
-                        dequant32_to_swizzled_row<QT, T16>(rr + QS::hdr_x(half), rr + QS::q0_x(half), rr + QS::q1_x(half), 0, 0, half,
-                                                           2 * (q & 1) + e, w_slot(n + e) + (uint32_t)(row * 64), (row >> 1) & 3, 0);
+                        dequant32_to_swizzled_row<QT, T16>(raw, half, q & 1, e, w_slot(n + e) + (uint32_t)(row * 64), (row >> 1) & 3, 0);
                     publish_pair(n);
                     if (dt == 0 && g2 == 0) trace(4, 2 * ui + pp);
                 }
@@ -305,10 +305,10 @@ __global__ void __launch_bounds__(kThreadsF, 1) k_umma_few(const __grid_constant
                 if (dt == 0 && g2 == 0) trace(3, ui >> 1);
                 const uint8_t *rr = smem + kOffRawF + ri * kRawStageBytes + row * BB;
                 const uint32_t w_addr = w_slot(n + st) + (uint32_t)(j * 4096 + r * 128);
+                Raw64<QT> raw;
+                raw.load(rr + hb * dev_half_step(QT), hb, j & 1);
 #pragma unroll
-                for (int e = 0; e < 2; e++)
-                    dequant32_to_swizzled_row<QT, T16>(rr + QS::hdr_x(hb), rr + QS::q0_x(hb), rr + QS::q1_x(hb), 0, 0, hb, 2 * (j & 1) + e,
-                                                       w_addr, r & 7, 4 * e);
+                for (int e = 0; e < 2; e++) dequant32_to_swizzled_row<QT, T16>(raw, hb, j & 1, e, w_addr, r & 7, 4 * e);
                 publish_pair(n);
                 if (dt == 0 && g2 == 0) trace(4, ui >> 1);
                 if (lane == 0) mbar_arrive(bar(kBRawEmpty + ri));
@@ -455,7 +455,7 @@ cudaError_t launch_umma_few(const UmmaLaunch &L, cudaStream_t s, const char **er
     const bool bwd = L.backward != 0;
     FewParams p;
     memset(&p, 0, sizeof(p));
-    p.tm_blk = bwd ? w->tm_blk_b : w->tm_blk_f;
+    p.tm_blk = bwd ? w->tm_blk : w->tm_blk_f;
     const int rows = L.rows > 0 ? L.rows : w->N;
     const int cols = bwd ? rows : w->K;       // contraction length of the activation operand
     if (!tmap_encode_2d(&p.tm_act, L.fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, L.act16, (uint64_t)cols,

@@ -13,7 +13,7 @@
 //   D[128 x tokens] (TMEM, fp32)  +=  Wtile[128 x 64] (SMEM, dequantized 16-bit)  x  act[tokens x 64]^T (SMEM via TMA)
 //
 // Warp roles (640 threads):
-//   warp 0        TMA producer of the packed half-super-blocks of W (raw bytes)
+//   warp 0        TMA producer of the packed super-blocks of W (raw bytes)
 //   warp 19       TMA producer of the 16-bit activation tiles
 //   warps 1, 18   tcgen05.mma issuers (one thread each, alternate stages, a turn token keeps the order fixed);
 //                 warp 1 owns the TMEM allocation
@@ -53,14 +53,19 @@ constexpr int kMaxTok = 512;       // tokens per CTA = TMEM columns
 constexpr int kAStageBytes = kTileW * kChunk * 2;   // 16 KiB
 constexpr int kNumA = 4;            // operand stages (dequantized weight tile + activation tile)
 // Shared memory of a CTA: [activation stages | dequantized weight stages | ring of packed weight blocks | barriers].
-// An activation stage holds XROWS token rows of 128 bytes (a kernel template parameter: 256 rows, or 128 in the
-// few-token variant).  Raw (still packed) weight blocks come from HBM, whose latency under load is several operand-stage
-// times (about 2.5 k clocks): the raw ring gets all the shared memory that is left, cut into as many stages as the
-// format's stage size allows (up to kMaxRaw) - 32 KB beside 256-row activation stages, 96 KB beside 128-row ones,
-// where nothing but the bytes in flight bounds the kernel.
+// An activation stage holds XROWS token rows of 128 bytes (a kernel template parameter: 256 rows, or 128 in the few-token
+// variant).  A raw stage is 128 weight rows x half a super-block (forward; see half_units in the kernel) or 64 rows x the half-blocks
+// that are the tile's 128 columns (backward), one piece of each packed row: the TMA unit takes a request per row piece, about 2
+// clocks for a 128-byte activation row and 4 to 5 for a packed one, and with a piece per field and half-block (4 per weight row
+// and 256 weights in Q4_K, 6 in Q6_K) the requests, not the tensor pipe, set the pace: 1150 - 1400 clocks per 64-deep stage at 512
+// tokens, where the MMAs take 1024, and 750 - 1150 at 131 tokens.  The dequant warps take their packed weights into registers
+// before they wait for the operand stage, so a raw stage is free again at once and few slots are enough beside 256-row
+// activation stages.  Clocks until the accumulator is complete, [18944, 3584], pieces per field -> one piece: Q6_K 131 tokens 74 k
+// -> 52 k forward, 74 k -> 54 k backward, 512 tokens 92 k -> 73 k and 82 k -> 75 k; Q4_K 131 tokens 38 k (44 k backward, was
+// 47 k), 512 tokens 73 k -> 69 k and 72 k.  (Whole super-blocks in the backward: twice the bytes in flight for the same work, 56 k instead of 47 k
+// clocks for Q4_K [18944, 3584] at 131 tokens.)
 constexpr int kOffX = 0;
 constexpr int kOffBar = kNumA * 32768 + kNumA * kAStageBytes + 32768;
-constexpr int kMaxRaw = 16;
 constexpr int kBarBytes = 512;
 constexpr int kDequantWarps = 16;   // four groups of 4
 constexpr int kThreads = 32 * (4 + kDequantWarps);   // + weight producer (0), two MMA issuers (1, 18), activation producer (19)
@@ -80,7 +85,7 @@ static_assert(kOffAbort + 4 <= kBarBytes, "barrier region too small");
 // each writes its own Y) or their output (backward: dX += sum over members of dY_m * W_m).
 constexpr int kMaxMembers = 3;
 struct Member {
-    CUtensorMap tm_hdr, tm_q0, tm_q1;   // packed weight bytes of this member
+    CUtensorMap tm_w;                   // packed weight bytes of this member (64-row boxes of whole or half super-blocks; 32 in the backward on paired rows), or fp16 rows
     CUtensorMap tm_act;                 // backward: this member's 16-bit dY; forward: member 0 holds the shared X
     float *out;                         // forward: this member's Y; backward: the shared dX (member 0 is read)
     const float *bias;
@@ -165,8 +170,7 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&v)[32], float *dst,
 //         shared memory saved goes to the ring of packed weight blocks).
 template <int QT, typename T16, bool BWD, bool PAIR, int MTOK, int XROWS>
 __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant__ Params p) {
-    using QS = QuantStage<QT>;
-    constexpr int H = QS::kHdrBytes, Q1 = QS::kQ1Bytes;
+    constexpr int BB = QT == kTypeF16 ? 16 : dev_block_bytes(QT);      // bytes of a super-block (fp16 rows have no raw stages)
     static_assert(XROWS == 256 || XROWS == 128, "activation stage: 256 or 128 token rows per CTA");
     constexpr int kXStageBytes = XROWS * 128;
     constexpr int kOffA = kOffX + kNumA * kXStageBytes;
@@ -176,19 +180,29 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
     // stage itself (128-byte swizzle = the tile image the dequantizer would have written)
     constexpr bool kDirect = QT == kTypeF16;
     constexpr int kRows = BWD ? 64 : 128;      // weight rows per raw stage
-    constexpr int kSub = BWD ? 1 : 2;          // operand stages produced per raw stage
+    // Forward units (a raw stage each): half super-blocks, but whole ones for Q4_K in a CTA pair - 512 tokens keep the TMA unit
+    // busy with activation rows, and fewer, longer weight rows leave it more (69 instead of 71 k clocks for [18944, 3584]); with up to
+    // 256 tokens three half-block stages in flight beat one whole one (38 instead of 49 k clocks at 131 tokens), and whole Q6_K
+    // stages are too big for either (512 tokens: 73 and 74 k, 131: 53 and 60 k).  sub = operand stages per unit (backward: 64 rows)
+    constexpr bool kHalf = BWD || !PAIR || QT != kTypeQ4K;
+    const bool half_units = kHalf || p.pair_hb != 0;
+    const int sub = BWD ? 1 : (half_units ? 2 : 4);
     constexpr int kNumX = kNumA;
-    constexpr int kRawStageBytes = (kRows * (H + 64 + Q1) + 1023) & ~1023;
+    constexpr int HB = dev_half_bytes(QT);
+    constexpr int kRawStageBytes = kDirect ? kRows * BB : kRows * (kHalf ? HB : BB);
+    const int rb_pitch = kHalf || p.pair_hb ? HB : BB;                 // bytes per weight row in a raw stage
     // Ring of packed blocks.  An mbarrier wait names a phase by its parity, so whoever waits on a barrier must visit
     // EVERY phase of it, one after the other (a waiter two phases behind would take the phase before last for the one
-    // it wants).  The dequant groups walk the raw stages with stride kStride (forward: two groups share a raw stage, the
-    // pairs alternate; backward: the four groups take every fourth stage).  Where kStride does not divide the number
+    // it wants).  The dequant groups walk the raw stages with stride kStride (forward on paired rows: two groups share a raw
+    // stage, the pairs alternate, otherwise every group takes its quarter of every stage; backward: the four groups take every
+    // fourth stage).  Where kStride does not divide the number
     // of slots, a slot gets one full / empty barrier pair per residue class r % kStride of the stages it holds: a
     // barrier (slot, class) then sees the stages r0, r0 + kLcm, r0 + 2 kLcm, ... and always the same waiters.  The
     // producer teams (stride kTeams, a divisor of kStride) wait for the stage that held the slot before.
     constexpr int kStride = BWD ? 4 : 2;
-    constexpr int kFit = kRawBudget / kRawStageBytes;
-    constexpr int kNumRaw = kFit < kMaxRaw ? (kFit < 1 ? 1 : kFit) : kMaxRaw;
+    constexpr int kFit = kDirect ? 1 : kRawBudget / kRawStageBytes;
+    constexpr int kNumRaw = kFit * kStride > kMaxRawBars ? kFit - kFit % kStride : kFit;
+    static_assert(kFit >= 1, "a raw stage fits");
     constexpr int kCls = kNumRaw % kStride == 0 ? 1 : kStride;
     constexpr int kLcm = kNumRaw % kStride == 0 ? kNumRaw : (kNumRaw % 2 == 0 ? 2 * kNumRaw : kStride * kNumRaw);
     constexpr int kTeams = kStride;      // weight-producer teams (three lanes each)
@@ -230,7 +244,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
     // columns costs its issuing thread about as much as a full-width one): the two issuers then work side by side, each
     // on its own set of partial accumulators (no turn token; every accumulator still receives its MMAs from one thread
     // in a fixed order, so results do not change from run to run).  Needs a main stage for either issuer.
-    const bool par = !PAIR && p.par_ok != 0 && acc_stride <= 128 && (u1 - u0) * (BWD ? 1 : 2) >= 2;
+    const bool par = !PAIR && p.par_ok != 0 && acc_stride <= 128 && (u1 - u0) * sub >= 2;
     const int n_acc_per = par ? (acc_stride <= 64 ? 4 : 2) : n_acc;      // partial accumulators per issuer
     const int n_acc_sum = par ? 2 * n_acc_per : n_acc;                   // ... that the epilogue adds up
     // forward: the member that owns this tile; backward: every CTA works on all members, unit by unit
@@ -254,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
     if (threadIdx.x == 0) {
         for (int i = 0; i < kNumRaw * kCls; i++) {
             mbar_init(bar(kBarRawFull + i), 1);
-            mbar_init(bar(kBarRawEmpty + i), BWD ? 4 : 8);       // one arrival per warp that read the stage
+            mbar_init(bar(kBarRawEmpty + i), BWD ? 4 : 4 * sub);       // one arrival per warp that read the stage
         }
         for (int i = 0; i < kNumA; i++) {
             // full: the (leader's) producer arrival carrying the TMA bytes + one arrival per dequant warp (of both CTAs)
@@ -269,8 +283,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
         *abort_flag = 0;
         fence_mbar_init();
         tma_prefetch_desc(&p.m[0].tm_act);
-        tma_prefetch_desc(&M.tm_hdr);
-        tma_prefetch_desc(&M.tm_q0);
+        tma_prefetch_desc(&M.tm_w);
     }
     if (warp == 1) {
         if (PAIR) {
@@ -352,7 +365,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                     int um = mi, rb = 0;
                     if (BWD) um = unit_member(u, rb);
                     const Member &W = p.m[um];
-                    for (int s = 0; s < kSub && ok; s++) {
+                    for (int s = 0; s < sub && ok; s++) {
                         ok = mbar_wait_bounded(bar(kBarEmpty + as.idx), as.phase ^ 1u, abort_flag, p.status, kCodeProducer + 1);
                         if (!ok) break;
                         const uint32_t adst = sbase + kOffA + as.idx * kAStageBytes;
@@ -362,27 +375,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                         if (BWD) {
                             // image `lane`: weight rows rb*64.., columns tile*128 + 64*lane ..
                             const int x = (tile * kTileW + 64 * lane) * 2, y = W.row_base + rb * 64;
-                            if (PAIR) tma_load_2d_pair(adst + lane * 8192, &W.tm_q0, x, y, fbar);
-                            else tma_load_2d(adst + lane * 8192, &W.tm_q0, x, y, fbar);
+                            if (PAIR) tma_load_2d_pair(adst + lane * 8192, &W.tm_w, x, y, fbar);
+                            else tma_load_2d(adst + lane * 8192, &W.tm_w, x, y, fbar);
                         } else {
                             const int x = (u * 2 + s) * 64 * 2, y = W.row_base + ltile * kTileW;
-                            if (PAIR) tma_load_2d_pair(adst, &W.tm_q0, x, y, fbar);
-                            else tma_load_2d(adst, &W.tm_q0, x, y, fbar);
+                            if (PAIR) tma_load_2d_pair(adst, &W.tm_w, x, y, fbar);
+                            else tma_load_2d(adst, &W.tm_w, x, y, fbar);
                         }
-                        if (lane == 0) trace(0, (u - u0) * kSub + s);
+                        if (lane == 0) trace(0, (u - u0) * sub + s);
                         as.advance(kNumA);
                     }
                 }
             }
-        } else if (lane < ((p.pair_hb || (!BWD && p.dual)) ? 6 : 3) * kTeams) {
-            // Teams of three lanes (lane 0 of a team arms the barrier and copies the headers, lanes 1 and 2 copy the
-            // quant regions); team t issues the raw stages r = t (mod kTeams).  Issuing a tiled copy holds the issuing
-            // thread for several hundred clocks: with one team the issue rate alone (one raw stage per ~800 clocks) paced
-            // the few-token shapes.  kTeams <= kNumRaw, so a team never waits for a slot whose previous stage is issued
-            // in the same round.
-            // (dual forward: six lanes, one per region and member; paired rows: one per region and row of a pair)
-            const int lpt = (p.pair_hb || (!BWD && p.dual)) ? 6 : 3;
-            const int team = lane / lpt, li = lane - lpt * team;
+        } else if (lane < 2 * kTeams) {
+            // Teams of two lanes, a copy each (lane 0 of a team arms the barrier): 64 of the 128 rows of a forward stage, the rows of
+            // one member of a dual forward, the half-blocks of one member of the row pairs; a backward stage is one copy of 64
+            // half-blocks (paired rows: two of 32).  Team t issues the raw stages r = t (mod kTeams): issuing a tiled copy holds the issuing thread for
+            // several hundred clocks.
+            const int team = lane >> 1, part = lane & 1;
+            const bool has_copy = !BWD || p.pair_hb || part == 0;
+            const int n_rows = BWD && !p.pair_hb ? 64 : kRows / 2;
             bool ok = true;
             for (int u = u0 + team; u < u1 && ok; u += kTeams) {
                 const int r = u - u0, ri = r % kNumRaw;
@@ -390,61 +402,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                 if (r >= kNumRaw)
                     ok = mbar_wait_bounded(bar(kBarRawEmpty + raw_bar(r - kNumRaw)), raw_phase(r - kNumRaw), abort_flag, p.status, kCodeProducer + 1);
                 if (!ok) break;
-                const uint32_t rdst = sbase + kOffRaw + ri * kRawStageBytes;
                 const uint32_t rbar = bar(kBarRawFull + raw_bar(r));
-                int sb, half, row0, um = mi, rb = 0;
-                if (BWD) {
-                    um = unit_member(u, rb);
-                    sb = tile >> 1; half = tile & 1; row0 = rb * 64;
-                } else {
-                    sb = u >> 1; half = u & 1; row0 = ltile * kTileW;
-                }
-                const Member &W = p.m[um];
-                if (p.pair_hb) {
-                    // half as many rows from either weight row of a pair: row h's boxes land behind row 0's in every region
-                    const int reg = li % 3, h = li / 3;
-                    const int hb = (BWD ? tile : u) + h * p.pair_hb, x = (hb >> 1) * QS::kBlockBytes, hf = hb & 1;
-                    const int region = reg == 0 ? 0 : (reg == 1 ? kRows * H : kRows * (H + 64));
-                    const int row_bytes = reg == 0 ? H : (reg == 1 ? 64 : Q1);
-                    if (li == 0) {
-                        mbar_arrive_expect_tx(rbar, (uint32_t)(kRows * (H + 64 + Q1)));
-                        if (lane == 0) trace(0, r / kTeams);
-                    }
-                    if (reg < 2 || Q1 > 0)
-                        tma_load_2d(rdst + region + h * (kRows / 2) * row_bytes, reg == 0 ? &W.tm_hdr : (reg == 1 ? &W.tm_q0 : &W.tm_q1),
-                                    x + (reg == 0 ? QS::hdr_x(hf) : (reg == 1 ? QS::q0_x(hf) : QS::q1_x(hf))), row0 >> 1, rbar);
-                    continue;
-                }
-                row0 += W.row_base;
-                const int xb = sb * QS::kBlockBytes;
-                if (!BWD && p.dual) {
-                    // 64 rows of either member (64-row boxes): member 1's rows land behind member 0's in every region
-                    const int reg = li % 3, mm = li / 3;
-                    const int region = reg == 0 ? 0 : (reg == 1 ? kRows * H : kRows * (H + 64));
-                    const int row_bytes = reg == 0 ? H : (reg == 1 ? 64 : Q1);
-                    const int x = xb + (reg == 0 ? QS::hdr_x(half) : (reg == 1 ? QS::q0_x(half) : QS::q1_x(half)));
-                    if (li == 0) {
-                        mbar_arrive_expect_tx(rbar, (uint32_t)(kRows * (H + 64 + Q1)));
-                        if (lane == 0) trace(0, r / kTeams);
-                    }
-                    if (reg < 2 || Q1 > 0) {
-                        const Member &Wm = p.m[mm];
-                        const CUtensorMap *tm = reg == 0 ? &Wm.tm_hdr : (reg == 1 ? &Wm.tm_q0 : &Wm.tm_q1);
-                        tma_load_2d(rdst + region + mm * 64 * row_bytes, tm, x, Wm.row_base + ltile * 64, rbar);
-                    }
-                    continue;
-                }
-                // one copy per region: the tensor maps handed to a forward launch have 128-row boxes, the backward
-                // ones 64-row boxes
-                if (li == 0) {
-                    mbar_arrive_expect_tx(rbar, (uint32_t)(kRows * (H + 64 + Q1)));
-                    tma_load_2d(rdst, &W.tm_hdr, xb + QS::hdr_x(half), row0, rbar);
+                if (part == 0) {
+                    mbar_arrive_expect_tx(rbar, (uint32_t)(kRows * rb_pitch));
                     if (lane == 0) trace(0, r / kTeams);
-                } else if (li == 1) {
-                    tma_load_2d(rdst + kRows * H, &W.tm_q0, xb + QS::q0_x(half), row0, rbar);
-                } else if (Q1 > 0) {
-                    tma_load_2d(rdst + kRows * (H + 64), &W.tm_q1, xb + QS::q1_x(half), row0, rbar);
                 }
+                if (!has_copy) continue;
+                int um = mi, rb = 0, x, row;
+                if (BWD) um = unit_member(u, rb);
+                if (!BWD && p.dual) um = part;
+                const int hb = (BWD ? tile : u) + part * p.pair_hb;      // half-block of the row (or pair of rows)
+                x = half_units ? (hb >> 1) * BB + (hb & 1) * dev_half_step(QT) : u * BB;
+                if (BWD) row = p.pair_hb ? rb * 32 : p.m[um].row_base + rb * 64;
+                else row = p.m[um].row_base + (p.dual || p.pair_hb ? ltile * 64 : ltile * kTileW + part * 64);
+                tma_load_2d(sbase + kOffRaw + ri * kRawStageBytes + part * n_rows * rb_pitch, &p.m[um].tm_w, x, row, rbar);
             }
         }
     } else if (warp == kActProducerWarp) {
@@ -457,12 +428,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                 int um = mi, rb = 0;
                 if (BWD) um = unit_member(u, rb);
                 const Member &W = p.m[um];
-                for (int s = 0; s < kSub && ok; s++) {
+                for (int s = 0; s < sub && ok; s++) {
                     ok = mbar_wait_bounded(bar(kBarEmpty + xs.idx), xs.phase ^ 1u, abort_flag, p.status, kCodeProducer + 2);
                     if (!ok) break;
-                    load_act_stage(BWD ? &W.tm_act : &p.m[0].tm_act, BWD ? rb * 64 : (u * 2 + s) * 64, sbase + kOffX + xs.idx * kXStageBytes,
+                    load_act_stage(BWD ? &W.tm_act : &p.m[0].tm_act, BWD ? rb * 64 : (u * sub + s) * 64, sbase + kOffX + xs.idx * kXStageBytes,
                                    bar(kBarFull + xs.idx), lane);
-                    if (lane == 0) trace(1, (u - u0) * kSub + s);
+                    if (lane == 0) trace(1, (u - u0) * sub + s);
                     xs.advance(kNumX);
                 }
             }
@@ -497,7 +468,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
                 tc_fence_after_sync();
                 return __all_sync(0xffffffffu, r);
             };
-            const int n_main = (u1 - u0) * kSub;
+            const int n_main = (u1 - u0) * sub;
             const int n_total = n_main + n_lora;
             // Everything an MMA needs is precomputed: the issuing thread is one thread, and at ~5 clocks per dependent
             // instruction a few dozen instructions per MMA would cost more than the MMA itself.
@@ -584,20 +555,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
             }
         };
         // operand stage n lives in A slot n % kNumA with phase (n / kNumA) & 1; raw stage i in slot i % kNumRaw.
-        // Runs r = 0, 1 of this thread: 32-weight group grp[r] of the row, written at dst_off[r] + chunk0[r].
-        // (row: its row in the raw stage, swz: swizzle phase of its row in the operand tile)
-        auto produce = [&](int n, const uint8_t *rs, int row, int swz, int half, const int (&grp)[2], const uint32_t (&dst_off)[2],
-                           const int (&chunk0)[2]) -> bool {
+        // This thread's 64 weights of operand stage n, from the half-block at hp: into registers, the raw stage is released, and
+        // then - once the operand slot is free - decoded as two 32-weight groups at dst + 16-byte chunks 4 e .. 4 e + 3.
+        using RawT = Raw64<QT == kTypeF16 ? kTypeQ4K : QT>;
+        auto produce = [&](int n, int raw_stage, const uint8_t *hp, int half, int pair, uint32_t dst_off, int swz) -> bool {
+            RawT raw;
+            raw.load(hp, half, pair);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(kBarRawEmpty + raw_bar(raw_stage)));
             const int ai = n % kNumA;
             if (!mbar_wait_bounded(bar(kBarEmpty + ai), ((uint32_t)(n / kNumA) & 1u) ^ 1u, abort_flag, p.status, kCodeDequant + 2))
                 return false;
             if (dt == 0 && g4 < 2) trace(3 + 3 * g4, n);
-            const uint32_t a_addr = sbase + kOffA + ai * kAStageBytes;
+            const uint32_t dst = sbase + kOffA + ai * kAStageBytes + dst_off;
+            if constexpr (!kDirect) {
 #pragma unroll
-            for (int r = 0; r < 2; r++)
-                dequant32_to_swizzled_row<QT, T16>(rs + row * H, rs + kRows * H + row * 64,
-                                                   rs + kRows * (H + 64) + row * (Q1 > 0 ? Q1 : 1), (row >> 1) & 3, (row >> 2) & 1,
-                                                   half, grp[r], a_addr + dst_off[r], swz, chunk0[r]);
+                for (int e = 0; e < 2; e++) dequant32_to_swizzled_row<QT, T16>(raw, half, pair, e, dst, swz, 4 * e);
+            }
             fence_proxy_async_smem();
             __syncwarp();
             signal_a_full(ai, 4);
@@ -607,43 +581,35 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
         if (kDirect) {
             // nothing to dequantize
         } else if (!BWD) {
-            // raw stage = 128 rows x half block = two operand stages (its 64-column halves); groups 0, 1 take the even
-            // raw stages, groups 2, 3 the odd ones; a thread owns one row of its group's half
-            // (paired rows: operand row dt is row dt >> 1 of the boxes of pair member dt & 1)
-            const int row = p.pair_hb ? (dt >> 1) + (dt & 1) * 64 : dt, sub = g4 & 1;
-            const int grp[2] = {2 * sub, 2 * sub + 1};
-            const int prow = p.dual ? dual_row(row) : dt;      // (prow & 7 == dt & 7)
-            const int hb0 = p.pair_hb && (dt & 1) ? p.pair_hb : 0;
-            const uint32_t dst_off[2] = {(uint32_t)(prow * 128), (uint32_t)(prow * 128)};
-            const int chunk0[2] = {0, 4};
-            for (int ui = g4 >> 1; ui < nu && ok; ui += 2) {
+            // a thread owns one row.  Whole rows: raw stage = 128 rows x a super-block = four operand stages, group g4 takes
+            // quarter g4 of every raw stage.  Paired rows: the stage holds half-block u of every row = two operand stages; groups 0, 1 take the even raw stages, groups 2, 3 the odd ones; operand row dt is row dt >> 1 of the
+            // boxes of pair member dt & 1.
+            const bool paired = p.pair_hb != 0;
+            const int row = paired ? (dt >> 1) + (dt & 1) * 64 : dt;
+            const int prow = p.dual ? dual_row(dt) : dt;      // (prow & 7 == dt & 7)
+            const int hb0 = paired && (dt & 1) ? p.pair_hb : 0;
+            for (int ui = half_units ? g4 >> 1 : 0; ui < nu && ok; ui += half_units ? 2 : 1) {
                 const int ri = ui % kNumRaw;
                 ok = mbar_wait_bounded(bar(kBarRawFull + raw_bar(ui)), raw_phase(ui), abort_flag, p.status, kCodeDequant + 1);
                 if (!ok) break;
-                if (dt == 0 && g4 < 2) trace(2 + 3 * g4, 2 * ui + sub);
-                const uint8_t *rs = smem + kOffRaw + ri * kRawStageBytes;
-                ok = produce(2 * ui + sub, rs, row, dt & 7, (u0 + ui + hb0) & 1, grp, dst_off, chunk0);
-                if (!ok) break;
-                if (lane == 0) mbar_arrive(bar(kBarRawEmpty + raw_bar(ui)));
+                if (dt == 0 && g4 < 2) trace(2 + 3 * g4, sub * ui + (g4 & (sub - 1)));
+                const int half = half_units ? (u0 + ui + hb0) & 1 : g4 >> 1;
+                const uint8_t *hp = smem + kOffRaw + ri * kRawStageBytes + row * rb_pitch + (half_units ? 0 : half * dev_half_step(QT));
+                ok = produce(sub * ui + (g4 & (sub - 1)), ui, hp, half, g4 & 1, (uint32_t)(prow * 128), dt & 7);
             }
         } else {
-            // raw stage = 64 rows x half block = one operand stage (two 64-column images); group g4 takes the stages
-            // ui = g4 (mod 4); a thread owns one row of one image
+            // raw stage = 64 rows x this tile's half-block = one operand stage (two 64-column images);
+            // group g4 takes the stages ui = g4 (mod 4); a thread owns one row of one image
             const int orow = dt & 63, im = dt >> 6;
             const int row = p.pair_hb ? (orow >> 1) + (orow & 1) * 32 : orow;
             const int hb0 = p.pair_hb && (orow & 1) ? p.pair_hb : 0;
-            const int grp[2] = {2 * im, 2 * im + 1};
-            const uint32_t dst_off[2] = {(uint32_t)(im * 8192 + orow * 128), (uint32_t)(im * 8192 + orow * 128)};
-            const int chunk0[2] = {0, 4};
             for (int ui = g4; ui < nu && ok; ui += 4) {
                 const int ri = ui % kNumRaw;
                 ok = mbar_wait_bounded(bar(kBarRawFull + raw_bar(ui)), raw_phase(ui), abort_flag, p.status, kCodeDequant + 1);
                 if (!ok) break;
                 if (dt == 0 && g4 < 2) trace(2 + 3 * g4, ui);
-                const uint8_t *rs = smem + kOffRaw + ri * kRawStageBytes;
-                ok = produce(ui, rs, row, orow & 7, (tile + hb0) & 1, grp, dst_off, chunk0);
-                if (!ok) break;
-                if (lane == 0) mbar_arrive(bar(kBarRawEmpty + raw_bar(ui)));
+                const uint8_t *hp = smem + kOffRaw + ri * kRawStageBytes + row * HB;
+                ok = produce(ui, ui, hp, (tile + hb0) & 1, im, (uint32_t)(im * 8192 + orow * 128), orow & 7);
             }
         }
         pdl_wait();      // from here on: the low-rank activations, the bias, the output
@@ -656,7 +622,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
             // both rounded to T16 here
             const Member &L = p.m[lora_m[lj]];
             const int rank_pad = (!BWD && p.dual) ? dual_pad[0] + dual_pad[1] : (L.rank + 15) & ~15;
-            const int n = (BWD ? 1 : 2) * nu + lj;
+            const int n = sub * nu + lj;
             const int ai = n % kNumA;
             if (ai != g4) continue;
             ok = mbar_wait_bounded(bar(kBarEmpty + ai), ((uint32_t)(n / kNumA) & 1u) ^ 1u, abort_flag, p.status, kCodeDequant + 3);
@@ -1009,68 +975,39 @@ cudaError_t umma_init_weight_maps(WeightDev *w, const char **err) {
         // fp16 rows: 128-byte-swizzled boxes of 64 columns x 128 rows (forward) / 64 rows (backward), written straight
         // into the operand stages
         if (w->K % 128 != 0 || w->row_bytes == 0) return cudaSuccess;
-        bool ok16 = encode_2d(&w->tm_q0_f, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
+        bool ok16 = encode_2d(&w->tm16_f, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
                               (uint64_t)w->row_bytes, 128, 128, CU_TENSOR_MAP_SWIZZLE_128B);
-        ok16 = ok16 && encode_2d(&w->tm_q0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
+        ok16 = ok16 && encode_2d(&w->tm16_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
                                  (uint64_t)w->row_bytes, 128, 64, CU_TENSOR_MAP_SWIZZLE_128B);
         if (!ok16) {
             if (err) *err = "cuTensorMapEncodeTiled failed for an fp16 weight tensor";
             return cudaErrorInvalidValue;
         }
-        w->tm_hdr = w->tm_q1 = w->tm_q0;
-        w->tm_hdr_f = w->tm_q1_f = w->tm_q0_f;
         w->tma_ok = true;
         return cudaSuccess;
     }
     if (w->qtype != kTypeQ4K && w->qtype != kTypeQ6K) return cudaSuccess;
-    const int H = w->qtype == kTypeQ4K ? 16 : 32;
+    const uint32_t bb = (uint32_t)dev_block_bytes(w->qtype), hb = (uint32_t)dev_half_bytes(w->qtype);
     if (w->K % 256 == 128 && w->N % 2 == 0) {
-        // two weight rows are a whole number of super-blocks: maps over [N / 2, 2 K], 64-row boxes (forward: 64 rows of either
-        // member of the pairs per stage) and 32-row boxes (backward), the latter in the *_f maps
-        const uint64_t rb = (uint64_t)(w->K / 128) * dev_block_bytes(w->qtype), rows = (uint64_t)w->N / 2;
-        bool okp = rb % 16 == 0;
-        for (int f = 0; f < 2; f++) {
-            const uint32_t box = f ? 32 : 64;
-            okp = okp && encode_2d(f ? &w->tm_hdr_f : &w->tm_hdr, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, rb, rows, rb, H, box, CU_TENSOR_MAP_SWIZZLE_NONE);
-            okp = okp && encode_2d(f ? &w->tm_q0_f : &w->tm_q0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, rb, rows, rb, 64, box, CU_TENSOR_MAP_SWIZZLE_64B);
-            if (w->qtype == kTypeQ6K)
-                okp = okp && encode_2d(f ? &w->tm_q1_f : &w->tm_q1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, rb, rows, rb, 32, box, CU_TENSOR_MAP_SWIZZLE_32B);
-        }
+        // two weight rows are a whole number of super-blocks: maps over [N / 2, 2 K], half-block boxes of 64 rows (forward: 64
+        // rows of either member of the pairs per stage) and of 32 rows (backward)
+        const uint64_t rb = (uint64_t)(w->K / 128) * bb, rows = (uint64_t)w->N / 2;
+        const bool okp = encode_2d(&w->tm_half, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, rb, rows, rb, hb, 64, CU_TENSOR_MAP_SWIZZLE_NONE) &&
+                         encode_2d(&w->tm_half_p, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, rb, rows, rb, hb, 32, CU_TENSOR_MAP_SWIZZLE_NONE);
         if (!okp) return cudaSuccess;      // the exact kernels take it
-        if (w->qtype == kTypeQ4K) {
-            w->tm_q1 = w->tm_q0;
-            w->tm_q1_f = w->tm_q0_f;
-        }
         w->pair_hb = w->K / 128;
         w->tma_ok = true;
         return cudaSuccess;
     }
     if (w->K % 256 != 0 || w->row_bytes == 0) return cudaSuccess;   // other flat streams run on the exact kernels
-    bool ok = encode_2d(&w->tm_hdr, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
-                        (uint64_t)w->row_bytes, H, 64, CU_TENSOR_MAP_SWIZZLE_NONE);
-    ok = ok && encode_2d(&w->tm_hdr_f, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
-                         (uint64_t)w->row_bytes, H, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
-    ok = ok && encode_2d(&w->tm_q0_f, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
-                         (uint64_t)w->row_bytes, 64, 128, CU_TENSOR_MAP_SWIZZLE_64B);
-    if (w->qtype == kTypeQ6K)
-        ok = ok && encode_2d(&w->tm_q1_f, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
-                             (uint64_t)w->row_bytes, 32, 128, CU_TENSOR_MAP_SWIZZLE_32B);
-    else
-        w->tm_q1_f = w->tm_q0_f;
-    ok = ok && encode_2d(&w->tm_q0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
-                         (uint64_t)w->row_bytes, 64, 64, CU_TENSOR_MAP_SWIZZLE_64B);
-    if (w->qtype == kTypeQ6K)
-        ok = ok && encode_2d(&w->tm_q1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
-                             (uint64_t)w->row_bytes, 32, 64, CU_TENSOR_MAP_SWIZZLE_32B);
-    else
-        w->tm_q1 = w->tm_q0;
-    {   // whole super-blocks for the few-token tensor-core kernel
-        const uint32_t bb = w->qtype == kTypeQ4K ? (uint32_t)kQ4KBlockBytes : (uint32_t)kQ6KDevBlockBytes;
-        ok = ok && encode_2d(&w->tm_blk_f, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
-                             (uint64_t)w->row_bytes, bb, 256, CU_TENSOR_MAP_SWIZZLE_NONE);
-        ok = ok && encode_2d(&w->tm_blk_b, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N,
-                             (uint64_t)w->row_bytes, bb, 64, CU_TENSOR_MAP_SWIZZLE_NONE);
-    }
+    // whole super-blocks: 256-row boxes for the few-token tensor-core kernel, 64-row boxes for the forward's raw stages; halves for
+    // the backward's
+    bool ok = encode_2d(&w->tm_blk_f, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N, (uint64_t)w->row_bytes, bb, 256,
+                        CU_TENSOR_MAP_SWIZZLE_NONE);
+    ok = ok && encode_2d(&w->tm_blk, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N, (uint64_t)w->row_bytes, bb, 64,
+                         CU_TENSOR_MAP_SWIZZLE_NONE);
+    ok = ok && encode_2d(&w->tm_half, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w->data, (uint64_t)w->row_bytes, (uint64_t)w->N, (uint64_t)w->row_bytes, hb, 64,
+                         CU_TENSOR_MAP_SWIZZLE_NONE);
     // whole packed super-blocks of 16 rows for the few-token streaming kernel: two Q4_K blocks or one Q6_K block per row
     ok = ok && encode_2d(&w->tm_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, w->data, (uint64_t)w->row_bytes / 4, (uint64_t)w->N,
                          (uint64_t)w->row_bytes, w->qtype == kTypeQ4K ? 72 : 56, 16, CU_TENSOR_MAP_SWIZZLE_NONE);
@@ -1083,21 +1020,21 @@ cudaError_t umma_init_weight_maps(WeightDev *w, const char **err) {
 }
 
 static int eff_rows(const UmmaLaunch &L) { return L.rows > 0 ? L.rows : L.w->N; }
+// contraction units of a forward: half super-blocks, or whole ones (see half_units in the kernel)
+static bool half_units(const WeightDev *w, bool pair) { return !pair || w->qtype != kTypeQ4K || w->pair_hb; }
+static int fwd_units(const WeightDev *w, bool pair) { return half_units(w, pair) ? w->K / 128 : w->K / 256; }
 
-static int pick_splits(int tiles, int units, int T, int sm_count) {
+// at least four (backward: two) 64-deep operand stages per split
+static int pick_splits(int tiles, int max_splits, int T, int sm_count) {
     const int chunks = (T + kMaxTok - 1) / kMaxTok;
     int s = sm_count / (tiles * chunks > 0 ? tiles * chunks : 1);
-    const int cap = units / 2 > 1 ? units / 2 : 1;
-    if (s > cap) s = cap;
-    if (s < 1) s = 1;
-    if (s > units) s = units;
-    return s;
+    if (s > max_splits) s = max_splits;
+    return s < 1 ? 1 : s;
 }
 
 int umma_pick_splits(const WeightDev *w, int backward, int T, int sm_count) {
     const int tiles = backward ? w->K / kTileW : (w->N + kTileW - 1) / kTileW;
-    const int units = backward ? (w->N + 63) / 64 : w->K / 128;
-    return pick_splits(tiles, units, T, sm_count);
+    return pick_splits(tiles, backward ? (w->N + 63) / 64 / 2 : w->K / 256, T, sm_count);
 }
 
 bool umma_group_ok(const UmmaLaunch *m, int n) {
@@ -1173,7 +1110,7 @@ int umma_group_splits(const UmmaLaunch *m, int n, int sm_count) {
             units = w->K / 128;
         }
     }
-    return pick_splits(tiles, units, m[0].T, sm_count);
+    return pick_splits(tiles, units / 2, m[0].T, sm_count);
 }
 
 // Members share T, math mode, direction, in_features and quantization type (umma_group_ok).  Forward: the activation
@@ -1255,11 +1192,7 @@ cudaError_t launch_umma_group(const UmmaLaunch *m, int n, cudaStream_t s, const 
         const UmmaLaunch &L = m[j];
         const WeightDev *w = L.w;
         Member &M = p.m[j];
-        // (64-row boxes: the backward's raw stages, and the dual forward's two half-tiles; paired rows: half of each)
-        const bool small_box = w->pair_hb ? !bwd : (bwd || dual);
-        M.tm_hdr = small_box ? w->tm_hdr : w->tm_hdr_f;
-        M.tm_q0 = small_box ? w->tm_q0 : w->tm_q0_f;
-        M.tm_q1 = small_box ? w->tm_q1 : w->tm_q1_f;
+        M.tm_w = w->qtype == kTypeF16 ? (bwd ? w->tm16_b : w->tm16_f) : (bwd && w->pair_hb ? w->tm_half_p : (bwd || half_units(w, pair) ? w->tm_half : w->tm_blk));
         const int rows = eff_rows(L);
         M.row_base = L.row_base;
         if (bwd || j == 0) {
@@ -1308,7 +1241,7 @@ cudaError_t launch_umma_group(const UmmaLaunch *m, int n, cudaStream_t s, const 
     p.trace = (long long *)L0.trace;
     p.T = L0.T;
     p.K = L0.w->K;
-    p.units = bwd ? first : L0.w->K / 128;
+    p.units = bwd ? first : fwd_units(L0.w, pair);
     p.splits = L0.splits < 1 ? 1 : (L0.splits > p.units ? p.units : L0.splits);
     if (dual) {
         p.splits = 1;
