@@ -140,7 +140,8 @@ template <int WQ, int WK>
 constexpr int kFwdSmem = 16 * WQ * SD + WK * 4 * kTile;
 template <typename T16, int WQ, int WK>
 __global__ void __launch_bounds__(32 * WQ * WK, 1) k_attn_fwd(const uint16_t *__restrict__ q, const uint16_t *__restrict__ k, const uint16_t *__restrict__ v,
-                                                              float *__restrict__ out, float *__restrict__ lse2, int T, int HQ, int HK) {
+                                                              float *__restrict__ out, uint16_t *__restrict__ out16, float *__restrict__ lse2, int T,
+                                                              int HQ, int HK) {
     constexpr int BQ = 16 * WQ, NG = 32 * WQ;      // queries per block, threads per group
     pdl_wait();
     pdl_trigger();
@@ -306,6 +307,11 @@ __global__ void __launch_bounds__(32 * WQ * WK, 1) k_attn_fwd(const uint16_t *__
         float *dst = out + (int64_t)row[r] * ldq + h * D;
 #pragma unroll
         for (int n = 0; n < D / 8; n++) *reinterpret_cast<float2 *>(dst + n * 8 + 2 * t4) = make_float2(o[n][2 * r] * inv, o[n][2 * r + 1] * inv);
+        if (out16) {      // the operand of the output projection: no cast pass has to read the fp32 copy back
+            uint16_t *d16 = out16 + (int64_t)row[r] * ldq + h * D;
+#pragma unroll
+            for (int n = 0; n < D / 8; n++) *reinterpret_cast<uint32_t *>(d16 + n * 8 + 2 * t4) = pack2<T16>(o[n][2 * r] * inv, o[n][2 * r + 1] * inv);
+        }
         if (t4 == 0) lse2[(int64_t)h * T + row[r]] = m[r] + log2f(l[r]);
     }
 }
@@ -667,14 +673,14 @@ int check_shape(int T, int HQ, int HK, int Dh, const char *who) {
 size_t a256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 template <typename T16>
-int forward16(gt_engine *e, const uint16_t *q, const uint16_t *k, const uint16_t *v, float *out, float *lse, int T, int HQ, int HK) {
+int forward16(gt_engine *e, const uint16_t *q, const uint16_t *k, const uint16_t *v, float *out, uint16_t *out16, float *lse, int T, int HQ, int HK) {
     // 128-query tiles where they give every SM a block; below that the chain of key tiles is what counts (4 x 2 against 8 x 1:
     // 15.6 / 19.7 us at 512 tokens and 28 heads, 18.5 / 27.9 at 777 and 8, but 79 / 69 at 1999 and 16)
     const int big = (T + 127) / 128;
     if (big * HQ >= e->sm_count)
-        GT_LAUNCH(e, launch_k(k_attn_fwd<T16, 8, 1>, dim3(HQ, big), dim3(256), kFwdSmem<8, 1>, e->stream, q, k, v, out, lse, T, HQ, HK));
+        GT_LAUNCH(e, launch_k(k_attn_fwd<T16, 8, 1>, dim3(HQ, big), dim3(256), kFwdSmem<8, 1>, e->stream, q, k, v, out, out16, lse, T, HQ, HK));
     else
-        GT_LAUNCH(e, launch_k(k_attn_fwd<T16, 4, 2>, dim3(HQ, (T + 63) / 64), dim3(256), kFwdSmem<4, 2>, e->stream, q, k, v, out, lse, T, HQ, HK));
+        GT_LAUNCH(e, launch_k(k_attn_fwd<T16, 4, 2>, dim3(HQ, (T + 63) / 64), dim3(256), kFwdSmem<4, 2>, e->stream, q, k, v, out, out16, lse, T, HQ, HK));
     return GT_OK;
 }
 template <typename T16>
@@ -705,12 +711,14 @@ int attention_operands_on_device(gt_engine *e, const float *q, const float *k, c
     return GT_OK;
 }
 
-int attention_forward16_on_device(gt_engine *e, const void *q16, const void *k16, const void *v16, float *out, float *lse, int T, int HQ, int HK, int Dh) {
+int attention_forward16_on_device(gt_engine *e, const void *q16, const void *k16, const void *v16, float *out, float *lse, int T, int HQ, int HK, int Dh,
+                                  void *out16) {
     int rc = check_shape(T, HQ, HK, Dh, "attention forward");
     if (rc == GT_OK) rc = attn_init();
     if (rc != GT_OK) return rc;
     const uint16_t *q = (const uint16_t *)q16, *k = (const uint16_t *)k16, *v = (const uint16_t *)v16;
-    return e->math_mode == GT_MATH_BF16 ? forward16<__nv_bfloat16>(e, q, k, v, out, lse, T, HQ, HK) : forward16<__half>(e, q, k, v, out, lse, T, HQ, HK);
+    return e->math_mode == GT_MATH_BF16 ? forward16<__nv_bfloat16>(e, q, k, v, out, (uint16_t *)out16, lse, T, HQ, HK)
+                                          : forward16<__half>(e, q, k, v, out, (uint16_t *)out16, lse, T, HQ, HK);
 }
 
 // scratch of a backward: delta [HQ, T], dO16 [T, HQ, D], the per-query-head dk / dv workspace [HQ, T, D] x 2; and, for the calls

@@ -125,19 +125,40 @@ size_t low_bytes(const gt_adapter *a, int T) { return ((size_t)T * a->rank * siz
 float *low_of(const gt_adapter *a) { return (float *)a->low.p; }
 float *dlow_of(const gt_adapter *a, int T) { return (float *)((char *)a->low.p + low_bytes(a, T)); }
 
-// low_j = X * A_j for every listed adapter (they share X), and optionally the 16-bit copy of X.  One memset per
-// adapter clears low (the warp-MMA kernel sums into it) and dLow of the same step; one kernel pass reads X.
-int compute_low(gt_engine *e, gt_adapter *const *ads, int n, const float *Xd, void *x16, int fp16, int T, int K,
-                const RowFill *fills = nullptr, int n_fills = 0) {
-    LoraXaJob jobs[kMaxGroup];
+int clear_lows(gt_engine *e, gt_adapter *const *ads, int n, int T) {
+    std::vector<ClearBuf> bufs((size_t)n);
+    for (int j = 0; j < n; j++) {
+        GT_CUDA(ads[j]->low.reserve(2 * low_bytes(ads[j], T)));
+        bufs[(size_t)j] = ClearBuf{ads[j]->low.p, 2 * low_bytes(ads[j], T)};
+        ads[j]->zeroed_T = T;
+    }
+    GT_LAUNCH(e, launch_clear(bufs.data(), n, e->stream));
+    return GT_OK;
+}
+// The same for the adapters of one group, but for those that were cleared ahead.
+int zero_low(gt_engine *e, gt_adapter *const *ads, int n, int T) {
+    ClearBuf bufs[kMaxGroup];
+    int nb = 0;
     for (int j = 0; j < n; j++) {
         gt_adapter *a = ads[j];
         GT_CUDA(a->low.reserve(2 * low_bytes(a, T)));
-        GT_CUDA(cudaMemsetAsync(a->low.p, 0, 2 * low_bytes(a, T), e->stream));
+        if (a->zeroed_T != T) bufs[nb++] = ClearBuf{a->low.p, 2 * low_bytes(a, T)};
+        a->zeroed_T = 0;
         a->low_T = T;
         a->dlow_clean = true;
-        jobs[j] = LoraXaJob{a->A, low_of(a), a->rank};
     }
+    if (nb) GT_LAUNCH(e, launch_clear(bufs, nb, e->stream));
+    return GT_OK;
+}
+
+// low_j = X * A_j for every listed adapter (they share X), and optionally the 16-bit copy of X.  low (the warp-MMA kernel
+// sums into it) and dLow of the same step are cleared first; one kernel pass reads X.
+int compute_low(gt_engine *e, gt_adapter *const *ads, int n, const float *Xd, void *x16, int fp16, int T, int K,
+                const RowFill *fills = nullptr, int n_fills = 0) {
+    LoraXaJob jobs[kMaxGroup];
+    int rc = zero_low(e, ads, n, T);
+    if (rc != GT_OK) return rc;
+    for (int j = 0; j < n; j++) jobs[j] = LoraXaJob{ads[j]->A, low_of(ads[j]), ads[j]->rank};
     if (e->math_mode == GT_MATH_BF16) {
         GT_LAUNCH(e, launch_lora_xa_group(Xd, jobs, n, x16, K, fp16, T, K, fills, n_fills, e->stream));      // fills ride along
     } else {
@@ -149,17 +170,15 @@ int compute_low(gt_engine *e, gt_adapter *const *ads, int n, const float *Xd, vo
 }
 
 // The same from an X that already exists as bf16 [T, K] (bf16 mode only): low_j = X16 * A_j, no copy is written.
+// keep: a low_j of this T that is in place stays.
 int compute_low16(gt_engine *e, gt_adapter *const *ads, int n, const void *X16, int T, int K, const RowFill *fills = nullptr,
-                  int n_fills = 0) {
+                  int n_fills = 0, bool keep = false) {
+    for (int j = 0; j < n; j++) keep = keep && ads[j]->low.p && ads[j]->low_T == T;
+    if (keep) n = 0;
     LoraXaJob jobs[kMaxGroup];
-    for (int j = 0; j < n; j++) {
-        gt_adapter *a = ads[j];
-        GT_CUDA(a->low.reserve(2 * low_bytes(a, T)));
-        GT_CUDA(cudaMemsetAsync(a->low.p, 0, 2 * low_bytes(a, T), e->stream));
-        a->low_T = T;
-        a->dlow_clean = true;
-        jobs[j] = LoraXaJob{a->A, low_of(a), a->rank};
-    }
+    int rc = zero_low(e, ads, n, T);
+    if (rc != GT_OK) return rc;
+    for (int j = 0; j < n; j++) jobs[j] = LoraXaJob{ads[j]->A, low_of(ads[j]), ads[j]->rank};
     for (int j = 0; j < n_fills; j++) GT_LAUNCH(e, launch_fill_rows(fills[j].dst, fills[j].bias, T, fills[j].N, e->stream));
     if (n) GT_LAUNCH(e, launch_lora_xa16_group(X16, K, jobs, n, T, K, e->stream));
     return GT_OK;
@@ -174,6 +193,11 @@ bool group_tensor_ok(const gt_engine *e, int n, const gt_weight *const *w) {
     for (int j = 0; j < n; j++)
         if (!tensor_path(e, w[j]) || w[j]->dev.K != w[0]->dev.K) return false;      // quantization types may differ (Q4_K_M mixes)
     return true;
+}
+
+// bf16 mode, tensor path, more tokens than the few-token kernels take (they stage fp32 activations themselves), 16-byte rows.
+bool group_x16_ok(const gt_engine *e, int n, const gt_weight *const *w, int T) {
+    return e->math_mode == GT_MATH_BF16 && T > 64 && group_tensor_ok(e, n, w) && w[0]->dev.K % 8 == 0;
 }
 
 // Few tokens (bf16 mode): the projections are bound by streaming the packed weights, which the warp-level kernel does
@@ -314,7 +338,7 @@ int forward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adap
     for (int j = 0; j < n; j++)
         if (lora[j]) with[n_with++] = ad[j];
     if (x16_ready) {
-        int rc = compute_low16(e, with, n_with, x16_ready, T, K, fills, n_fills);
+        int rc = compute_low16(e, with, n_with, x16_ready, T, K, fills, n_fills, (flags & kFlagKeepLow) != 0);
         if (rc != GT_OK) return rc;
         for (int j = 0; j < n; j++)
             if (lora[j]) m[j].lora_act = low_of(ad[j]);
@@ -651,7 +675,7 @@ bool ffn_dual_ok(const gt_engine *e, const gt_weight *const *w, gt_adapter *cons
 }
 
 int ffn_forward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *const *ad, const float *Xd, float *gate_d, float *up_d,
-                       float *hidden_d, float *Yd, int T, int flags, void *hidden16) {
+                       float *hidden_d, float *Yd, int T, int flags, void *hidden16, const void *X16) {
     const int F = w[0]->dev.N;
     const size_t bf = (size_t)T * F * sizeof(float);
     const bool fold = ffn_hidden16_ok(e, w, T);
@@ -661,12 +685,12 @@ int ffn_forward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *cons
         // gate and up themselves are written where the caller gave a place for them (a backward needs them; a forward
         // pass whose state is recomputed later does not).
         float *gu[2] = {gate_d, up_d};
-        int rc = forward_group_device(e, 2, w, ad, Xd, gu, T, flags, nullptr, hidden16);
+        int rc = forward_group_device(e, 2, w, ad, Xd, gu, T, flags, X16, hidden16);
         if (rc != GT_OK || !Yd) return rc;
         float *yd = Yd;
         return forward_group_device(e, 1, w + 2, ad ? ad + 2 : nullptr, nullptr, &yd, T, flags, hidden16);
     }
-    if (Yd && !hidden16 && w[0]->dev.N == w[1]->dev.N && decode_ok(e, 2, true, w, Xd, T)) {
+    if (Yd && !hidden16 && !X16 && w[0]->dev.N == w[1]->dev.N && decode_ok(e, 2, true, w, Xd, T)) {
         // few tokens: gate | up and the product in one launch, gate and up written only where the caller wants them
         float *h = hidden_d;
         if (!h) {
@@ -692,7 +716,7 @@ int ffn_forward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *cons
         }
     }
     float *gu[2] = {bufs[0], bufs[1]};
-    int rc = forward_group_device(e, 2, w, ad, Xd, gu, T, flags);
+    int rc = forward_group_device(e, 2, w, ad, Xd, gu, T, flags, X16);
     if (rc != GT_OK) return rc;
     float *yd = Yd;
     if (!Yd) {
@@ -725,7 +749,7 @@ int ffn_forward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *cons
 // dX (+)= dGate * W_gate + dUp * W_up (+ adapters); adapter gradients accumulate.  Device tensors.
 int ffn_backward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *const *ad, const float *dYd, const float *Xd,
                         const float *gate_d, const float *up_d, const float *hidden_d, float *dXd, int T, int flags,
-                        const void *hidden16) {
+                        const void *hidden16, const void *X16) {
     const int F = w[0]->dev.N;
     const size_t bf = (size_t)T * F * sizeof(float);
     if (hidden16 && !ffn_hidden16_ok(e, w, T))
@@ -747,11 +771,11 @@ int ffn_backward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *con
         GT_LAUNCH(e, launch_swiglu_bwd16(dh, gate_d, up_d, (char *)e->dy16.p + off[0], (char *)e->dy16.p + off[1], (int64_t)T * F, e->sm_count,
                                          e->stream));
         const float *none[2] = {nullptr, nullptr};
-        return backward_group_device(e, 2, w, ad, none, Xd, dXd, T, flags, nullptr, true);
+        return backward_group_device(e, 2, w, ad, none, Xd, dXd, T, flags, X16, true);
     }
     GT_LAUNCH(e, launch_swiglu_bwd(dh, gate_d, up_d, dg, du, (int64_t)T * F, e->sm_count, e->stream));
     const float *dgu[2] = {dg, du};
-    return backward_group_device(e, 2, w, ad, dgu, Xd, dXd, T, flags);
+    return backward_group_device(e, 2, w, ad, dgu, Xd, dXd, T, flags, X16);
 }
 
 // the engine stream waits for the collectives begun on the side stream (gt_dp_allreduce_begin)

@@ -137,6 +137,7 @@ struct gt_adapter {
                                  // [low_T, rank] fp32 each
     int low_T = 0;
     bool dlow_clean = false;     // dLow is still all zero (cleared together with low, not yet summed into)
+    int zeroed_T = 0;            // low and dLow for this many tokens were cleared ahead of the pass that is being queued
     Scratch xkeep;               // host-buffer calls: device copy of the X of the last forward, for a backward that
     int xkeep_T = 0;             // reuses it (GT_FLAG_REUSE_LOW) instead of uploading X again
     Scratch moments;             // AdamW state [mA | vA | mB | vB], allocated and zeroed by the first optimizer step
@@ -157,14 +158,21 @@ int forward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adap
                          int T, int flags, const void *x16_ready = nullptr, void *dual_h16 = nullptr);
 int backward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adapter *const *ad, const float *const *dYd,
                           const float *Xd, float *dXd, int T, int flags, const void *X16 = nullptr, bool dy16_ready = false);
+// The group's input may be handed over as bf16 only (x16_ready forward, X16 backward).
+bool group_x16_ok(const gt_engine *e, int n, const gt_weight *const *w, int T);
+// With x16_ready: the adapters' X*A of an earlier forward of this pass on the same X is still in place and is not formed again
+// (the recomputed forward of a checkpointed block).
+constexpr int kFlagKeepLow = 1 << 30;
+// Clears low and dLow of the listed adapters for a pass over T tokens in one launch; the forward calls that follow find them zeroed.
+int clear_lows(gt_engine *e, gt_adapter *const *ads, int n, int T);
 // SiLU(gate) * up can be kept as bf16 only (hidden16: [T, ffn] bf16, hidden_d null) when ffn_hidden16_ok(): the SwiGLU pass
 // then writes the down projection's 16-bit operand itself and the adapter products of the down projection read that copy.
 bool ffn_hidden16_ok(const gt_engine *e, const gt_weight *const *w, int T);
 int ffn_forward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *const *ad, const float *Xd, float *gate_d, float *up_d,
-                       float *hidden_d, float *Yd, int T, int flags, void *hidden16 = nullptr);
+                       float *hidden_d, float *Yd, int T, int flags, void *hidden16 = nullptr, const void *X16 = nullptr);
 int ffn_backward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *const *ad, const float *dYd, const float *Xd,
                         const float *gate_d, const float *up_d, const float *hidden_d, float *dXd, int T, int flags,
-                        const void *hidden16 = nullptr);
+                        const void *hidden16 = nullptr, const void *X16 = nullptr);
 int join_comm(gt_engine *e);
 int allreduce_begin_locked(gt_engine *e, float *g_dev, int64_t count, float scale);
 // forget the captured step of every model of this engine (before the communicator its collectives belong to goes away)
@@ -178,7 +186,7 @@ int embedding_on_device(gt_engine *e, const gt_weight *w, const int *tokens, int
 int attention_operands_on_device(gt_engine *e, const float *q, const float *k, const float *v, void *q16, void *k16, void *v16, int T, int heads_q,
                                  int heads_kv, float rope_freq_base);
 int attention_forward16_on_device(gt_engine *e, const void *q16, const void *k16, const void *v16, float *out, float *lse, int T, int heads_q,
-                                  int heads_kv, int head_dim);
+                                  int heads_kv, int head_dim, void *out16 = nullptr);      // out16: a rounded copy of out as well
 int attention_backward16_on_device(gt_engine *e, const float *d_out, const void *q16, const void *k16, const void *v16, const float *out, const float *lse,
                                    float *dq, float *dk, float *dv, int T, int heads_q, int heads_kv, int head_dim);
 }  // namespace gt

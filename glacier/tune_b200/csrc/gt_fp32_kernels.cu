@@ -97,6 +97,36 @@ cudaError_t launch_cast16(const float *src, void *dst, int rows, int cols, int l
     return launch_k(k_cast16, dim3(blocks), dim3(256), 0, s, src, (uint16_t *)dst, rows, cols, ld_dst, fp16);
 }
 
+// Many small buffers in one launch (the adapters' summed products of a whole pass): a memset each costs more than a microsecond
+// and ends the overlap of the launches around it.
+struct ClearArgs {
+    uint4 *p[kClearBufs];
+    uint32_t n16[kClearBufs];
+};
+__global__ void __launch_bounds__(256) k_clear(const ClearArgs a) {
+    pdl_wait();
+    pdl_trigger();
+    uint4 *p = a.p[blockIdx.y];
+    const uint32_t n = a.n16[blockIdx.y];
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) p[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+cudaError_t launch_clear(const ClearBuf *bufs, int n, cudaStream_t s) {
+    for (int i0 = 0; i0 < n; i0 += kClearBufs) {
+        ClearArgs a{};
+        const int m = n - i0 < kClearBufs ? n - i0 : kClearBufs;
+        uint32_t most = 0;
+        for (int i = 0; i < m; i++) {
+            a.p[i] = (uint4 *)bufs[i0 + i].p;
+            a.n16[i] = (uint32_t)(bufs[i0 + i].bytes / 16);
+            most = a.n16[i] > most ? a.n16[i] : most;
+        }
+        const uint32_t want = (most + 1023) / 1024, cap = m > 16 ? 4 : 64;      // 16 KB a block, about 500 blocks at most
+        cudaError_t e = launch_k(k_clear, dim3(want < 1 ? 1 : (want > cap ? cap : want), (unsigned)m), dim3(256), (size_t)0, s, a);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 __global__ void k_fill_rows(float *__restrict__ Y, const float *__restrict__ bias, int T, int N) {
     pdl_wait();
     pdl_trigger();

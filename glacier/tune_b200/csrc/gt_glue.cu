@@ -286,12 +286,19 @@ __device__ __forceinline__ void block_sum2(float &a, float &b) {
 
 // One block per token row; the row (H <= 16 * 256 floats kept in registers, longer rows re-read) is read once.
 constexpr int kRowRegs = 16;
-__global__ void __launch_bounds__(256) k_rmsnorm_fwd(const float *__restrict__ x, const float *__restrict__ w, float *__restrict__ y, int H,
-                                                     float eps) {
+// y16 given: the row goes out rounded to bf16 there and y is not written (what reads a norm's output on the tensor path rounds it
+// anyway: an fp32 copy would be written, read back and cast).
+__device__ __forceinline__ void norm_store(float *yr, __nv_bfloat16 *yr16, int i, float v) {
+    if (yr16) yr16[i] = __float2bfloat16_rn(v);
+    else yr[i] = v;
+}
+__global__ void __launch_bounds__(256) k_rmsnorm_fwd(const float *__restrict__ x, const float *__restrict__ w, float *__restrict__ y,
+                                                     __nv_bfloat16 *__restrict__ y16, int H, float eps) {
     pdl_wait();
     pdl_trigger();
     const float *xr = x + (int64_t)blockIdx.x * H;
     float *yr = y + (int64_t)blockIdx.x * H;
+    __nv_bfloat16 *yr16 = y16 ? y16 + (int64_t)blockIdx.x * H : nullptr;
     float v[kRowRegs];
     float ss = 0.f, unused = 0.f;
 #pragma unroll
@@ -306,20 +313,22 @@ __global__ void __launch_bounds__(256) k_rmsnorm_fwd(const float *__restrict__ x
 #pragma unroll
     for (int j = 0; j < kRowRegs; j++) {
         const int i = threadIdx.x + j * 256;
-        if (i < H) yr[i] = v[j] * r * w[i];
+        if (i < H) norm_store(yr, yr16, i, v[j] * r * w[i]);
     }
-    for (int i = threadIdx.x + kRowRegs * 256; i < H; i += 256) yr[i] = xr[i] * r * w[i];
+    for (int i = threadIdx.x + kRowRegs * 256; i < H; i += 256) norm_store(yr, yr16, i, xr[i] * r * w[i]);
 }
 
 // sum = a + b (written out: the residual stream), y = RMSNorm(sum) * w: the residual add and the norm that follows it
 // in one pass (TransformerBlock.cs:518-528: x1 = x + o, then norm2X = RMSNorm(x1)).  The sum is formed once in fp32 and
 // both outputs use it, so the values equal the two separate kernels'.
 __global__ void __launch_bounds__(256) k_add_rmsnorm_fwd(const float *__restrict__ a, const float *__restrict__ b, const float *__restrict__ w,
-                                                         float *__restrict__ sum, float *__restrict__ y, int H, float eps) {
+                                                         float *__restrict__ sum, float *__restrict__ y, __nv_bfloat16 *__restrict__ y16, int H,
+                                                         float eps) {
     pdl_wait();
     pdl_trigger();
     const float *ar = a + (int64_t)blockIdx.x * H, *br = b + (int64_t)blockIdx.x * H;
     float *sr = sum + (int64_t)blockIdx.x * H, *yr = y + (int64_t)blockIdx.x * H;
+    __nv_bfloat16 *yr16 = y16 ? y16 + (int64_t)blockIdx.x * H : nullptr;
     float v[kRowRegs];
     float ss = 0.f, unused = 0.f;
 #pragma unroll
@@ -339,9 +348,9 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_fwd(const float *__restrict
 #pragma unroll
     for (int j = 0; j < kRowRegs; j++) {
         const int i = threadIdx.x + j * 256;
-        if (i < H) yr[i] = v[j] * r * w[i];
+        if (i < H) norm_store(yr, yr16, i, v[j] * r * w[i]);
     }
-    for (int i = threadIdx.x + kRowRegs * 256; i < H; i += 256) yr[i] = sr[i] * r * w[i];
+    for (int i = threadIdx.x + kRowRegs * 256; i < H; i += 256) norm_store(yr, yr16, i, sr[i] * r * w[i]);
 }
 
 // dx = r * g - x * r^3 * mean(g * x), g = dy * w (frozen weight)
@@ -436,15 +445,16 @@ cudaError_t launch_rope(float *q, float *k, int T, int heads_q, int heads_kv, in
     return launch_k(k_rope, dim3((unsigned)T), dim3(256), (size_t)0, s, q, k, T, heads_q, heads_kv, head_dim, freq_base, freq_scale, eff,
                     inverse ? -1.0f : 1.0f, vec);
 }
-cudaError_t launch_rmsnorm_fwd(const float *x, const float *w, float *y, int T, int H, float eps, cudaStream_t s) {
-    return launch_k(k_rmsnorm_fwd, dim3((unsigned)T), dim3(256), (size_t)0, s, x, w, y, H, eps);
+cudaError_t launch_rmsnorm_fwd(const float *x, const float *w, float *y, int T, int H, float eps, cudaStream_t s, void *y16) {
+    return launch_k(k_rmsnorm_fwd, dim3((unsigned)T), dim3(256), (size_t)0, s, x, w, y, (__nv_bfloat16 *)y16, H, eps);
 }
 cudaError_t launch_rmsnorm_bwd(const float *dy, const float *x, const float *w, const float *residual, float *dx, int T, int H, float eps,
                                cudaStream_t s) {
     return launch_k(k_rmsnorm_bwd, dim3((unsigned)T), dim3(256), (size_t)0, s, dy, x, w, residual, dx, H, eps);
 }
-cudaError_t launch_add_rmsnorm_fwd(const float *a, const float *b, const float *w, float *sum, float *y, int T, int H, float eps, cudaStream_t s) {
-    return launch_k(k_add_rmsnorm_fwd, dim3((unsigned)T), dim3(256), (size_t)0, s, a, b, w, sum, y, H, eps);
+cudaError_t launch_add_rmsnorm_fwd(const float *a, const float *b, const float *w, float *sum, float *y, int T, int H, float eps, cudaStream_t s,
+                                   void *y16) {
+    return launch_k(k_add_rmsnorm_fwd, dim3((unsigned)T), dim3(256), (size_t)0, s, a, b, w, sum, y, (__nv_bfloat16 *)y16, H, eps);
 }
 cudaError_t launch_adamw(const AdamwSeg *segs, int n, float lr, float beta1, float beta2, float eps, float weight_decay, int step,
                          int sm_count, cudaStream_t s) {
@@ -536,7 +546,7 @@ extern "C" int gt_rmsnorm_forward(gt_engine *eng, const float *x, const float *w
     const gt::EngineView ev = gt::engine_view(eng);
     std::lock_guard<std::mutex> lk(*static_cast<std::mutex *>(ev.mutex));
     cudaError_t ce = cudaSetDevice(ev.device);
-    if (ce == cudaSuccess) ce = gt::launch_k(k_rmsnorm_fwd, dim3((unsigned)T), dim3(256), (size_t)0, ev.stream, x, w, y, (int)H, eps);
+    if (ce == cudaSuccess) ce = gt::launch_k(k_rmsnorm_fwd, dim3((unsigned)T), dim3(256), (size_t)0, ev.stream, x, w, y, (__nv_bfloat16 *)nullptr, (int)H, eps);
     return ce == cudaSuccess ? GT_OK : cuda_fail("gt_rmsnorm_forward", ce);
 }
 

@@ -45,6 +45,13 @@ struct WeightDev {
 };
 
 // ---- CUDA-core kernels (gt_fp32_kernels.cu) -------------------------------------------------------------
+// zeroes up to any number of buffers (16-byte aligned, sizes multiples of 16) in launches of kClearBufs
+struct ClearBuf {
+    void *p;
+    size_t bytes;
+};
+constexpr int kClearBufs = 128;
+cudaError_t launch_clear(const ClearBuf *bufs, int n, cudaStream_t s);
 cudaError_t launch_q4k_repack(uint8_t *blocks, int64_t nblocks, cudaStream_t s);      // in place
 cudaError_t launch_q6k_repack(const uint8_t *gguf_blocks, uint8_t *dev_blocks, int64_t nblocks, cudaStream_t s);
 cudaError_t launch_dequant_rows(int qt, const uint8_t *w, int K, int64_t row0, int64_t nrows, float *out, cudaStream_t s);
@@ -246,12 +253,14 @@ cudaError_t launch_swiglu_bwd(const float *d_hidden, const float *gate, const fl
 cudaError_t launch_add(const float *a, const float *b, float *out, int64_t n, int sm_count, cudaStream_t s);
 cudaError_t launch_rope(float *q, float *k, int T, int heads_q, int heads_kv, int head_dim, float freq_base, float freq_scale, int rope_dim,
                         int inverse, cudaStream_t s);
-cudaError_t launch_rmsnorm_fwd(const float *x, const float *w, float *y, int T, int H, float eps, cudaStream_t s);
+// (y16 given: the norm goes out as bf16 there and y is not written)
+cudaError_t launch_rmsnorm_fwd(const float *x, const float *w, float *y, int T, int H, float eps, cudaStream_t s, void *y16 = nullptr);
 // dx = RMSNorm backward (+ residual, which may be null and may alias dx)
 cudaError_t launch_rmsnorm_bwd(const float *dy, const float *x, const float *w, const float *residual, float *dx, int T, int H, float eps,
                                cudaStream_t s);
 // sum = a + b (sum may alias a or b), y = RMSNorm(sum) * w
-cudaError_t launch_add_rmsnorm_fwd(const float *a, const float *b, const float *w, float *sum, float *y, int T, int H, float eps, cudaStream_t s);
+cudaError_t launch_add_rmsnorm_fwd(const float *a, const float *b, const float *w, float *sum, float *y, int T, int H, float eps, cudaStream_t s,
+                                   void *y16 = nullptr);
 
 // ---- launches with programmatic dependent launch (the kernel must call pdl_wait() before touching global memory).
 // On by default; environment GT_PDL=0 launches in plain stream order.

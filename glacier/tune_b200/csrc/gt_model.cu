@@ -27,8 +27,9 @@ namespace {
 enum { kQ = 0, kK, kV, kO, kGate, kUp, kDown, kProj };
 
 struct BlockState {      // what a block's backward needs from its forward
-    float *n1, *attn, *lse, *x1, *n2, *gate, *up, *hidden;
+    float *n1, *attn, *lse, *x1, *n2, *gate, *up, *hidden;      // n1, n2: bf16 values where their projections take them (Inputs16)
     void *q16, *k16, *v16;      // the attention's operands: q, k rotated (q scaled), v, rounded to 16 bits
+    void *attn16;               // attn as the output projection's bf16 operand
 };
 struct LayerDev {
     const gt_weight *w[kProj] = {};
@@ -93,6 +94,16 @@ int check_ready(const gt_model *m, const char *who) {
     return GT_OK;
 }
 
+// Which projections of a block take their input as bf16: then the norms and the attention write that alone (or as well: the
+// attention's backward reads the fp32 output too), and neither a cast nor the adapters' products read an fp32 tensor back.
+struct Inputs16 {
+    bool qkv, o, gu;
+};
+Inputs16 inputs16(const gt_model *m, int l, int T) {
+    const LayerDev &L = m->layers[l];
+    return {group_x16_ok(m->eng, 3, L.w + kQ, T), group_x16_ok(m->eng, 1, L.w + kO, T), group_x16_ok(m->eng, 2, L.w + kGate, T)};
+}
+
 // One block forward on the engine stream; s receives the state.  n1_ready: s.n1 already holds RMSNorm(x_in) (the block
 // before wrote it together with its output).  next_norm / next_n1 (may be null): the norm weight and destination of
 // the norm that follows this block's output - the next block's attention norm or the model's output norm - computed
@@ -106,27 +117,33 @@ int block_forward(gt_model *m, int l, const float *x_in, float *x_out, BlockStat
     const gt_model_config &c = m->cfg;
     const LayerDev &L = m->layers[l];
     const int H = c.hidden;
-    if (!n1_ready) GT_LAUNCH(e, launch_rmsnorm_fwd(x_in, L.norm1, s.n1, T, H, c.rms_eps, e->stream));
+    const Inputs16 i16 = inputs16(m, l, T);
+    const int keep = x_out ? 0 : kFlagKeepLow;      // recomputed: the adapters' X*A are still there from the forward pass
+    if (!n1_ready) GT_LAUNCH(e, launch_rmsnorm_fwd(x_in, L.norm1, s.n1, T, H, c.rms_eps, e->stream, i16.qkv ? s.n1 : nullptr));
     float *qkv[3] = {m->q, m->k, m->v};
-    int rc = forward_group_device(e, 3, L.w + kQ, L.ad + kQ, s.n1, qkv, T, 0);
+    int rc = forward_group_device(e, 3, L.w + kQ, L.ad + kQ, s.n1, qkv, T, keep, i16.qkv ? s.n1 : nullptr);
     if (rc != GT_OK) return rc;
     // RoPE on q and k, and the 16-bit operands of the attention and of its backward, in one pass
     rc = attention_operands_on_device(e, m->q, m->k, m->v, s.q16, s.k16, s.v16, T, c.n_heads, c.n_kv_heads, c.rope_theta);
-    if (rc == GT_OK) rc = attention_forward16_on_device(e, s.q16, s.k16, s.v16, s.attn, s.lse, T, c.n_heads, c.n_kv_heads, c.head_dim);
+    if (rc == GT_OK) rc = attention_forward16_on_device(e, s.q16, s.k16, s.v16, s.attn, s.lse, T, c.n_heads, c.n_kv_heads, c.head_dim,
+                                                     i16.o ? s.attn16 : nullptr);
     if (rc != GT_OK) return rc;
     float *o = m->tmp_h;
-    rc = forward_group_device(e, 1, L.w + kO, L.ad + kO, s.attn, &o, T, 0);
+    rc = forward_group_device(e, 1, L.w + kO, L.ad + kO, s.attn, &o, T, keep, i16.o ? s.attn16 : nullptr);
     if (rc != GT_OK) return rc;
-    GT_LAUNCH(e, launch_add_rmsnorm_fwd(x_in, o, L.norm2, s.x1, s.n2, T, H, c.rms_eps, e->stream));      // x1 = x + o; n2 = norm(x1)
+    // x1 = x + o; n2 = norm(x1)
+    GT_LAUNCH(e, launch_add_rmsnorm_fwd(x_in, o, L.norm2, s.x1, s.n2, T, H, c.rms_eps, e->stream, i16.gu ? s.n2 : nullptr));
     const gt_weight *fw[3] = {L.w[kGate], L.w[kUp], L.w[kDown]};
     gt_adapter *fa[3] = {L.ad[kGate], L.ad[kUp], L.ad[kDown]};
     // SiLU(gate) * up is kept as bf16 only where the engine can work from that (the buffer is sized for fp32 either way)
     const bool h16 = ffn_hidden16_ok(e, fw, T);
     const bool drop_gu = !keep_gu && h16 && x_out;      // (without the 16-bit product the SwiGLU pass reads them from the state)
     rc = ffn_forward_device(e, fw, fa, s.n2, drop_gu ? nullptr : s.gate, drop_gu ? nullptr : s.up, h16 ? nullptr : s.hidden,
-                            x_out ? m->tmp_h : nullptr, T, 0, h16 ? (void *)s.hidden : nullptr);
+                            x_out ? m->tmp_h : nullptr, T, keep, h16 ? (void *)s.hidden : nullptr, i16.gu ? s.n2 : nullptr);
     if (rc != GT_OK || !x_out) return rc;
-    if (next_norm && next_n1) GT_LAUNCH(e, launch_add_rmsnorm_fwd(s.x1, m->tmp_h, next_norm, x_out, next_n1, T, H, c.rms_eps, e->stream));
+    const bool next16 = l + 1 < (int)m->layers.size() && inputs16(m, l + 1, T).qkv;
+    if (next_norm && next_n1)
+        GT_LAUNCH(e, launch_add_rmsnorm_fwd(s.x1, m->tmp_h, next_norm, x_out, next_n1, T, H, c.rms_eps, e->stream, next16 ? next_n1 : nullptr));
     else GT_LAUNCH(e, launch_add(s.x1, m->tmp_h, x_out, (int64_t)T * H, e->sm_count, e->stream));
     return GT_OK;
 }
@@ -142,19 +159,20 @@ int block_backward(gt_model *m, int l, const float *d_out, const float *x_in, co
     gt_adapter *fa[3] = {L.ad[kGate], L.ad[kUp], L.ad[kDown]};
     // A. FFN: down, SwiGLU, gate | up -> dNorm2X; RMSNorm2 backward + residual: dX1 = dOut + dNorm(dNorm2X)
     const bool h16 = ffn_hidden16_ok(e, fw, T);
+    const Inputs16 i16 = inputs16(m, l, T);
     int rc = ffn_backward_device(e, fw, fa, d_out, s.n2, s.gate, s.up, h16 ? nullptr : s.hidden, m->dn, T, flags,
-                                 h16 ? (const void *)s.hidden : nullptr);
+                                 h16 ? (const void *)s.hidden : nullptr, i16.gu ? s.n2 : nullptr);
     if (rc != GT_OK) return rc;
     GT_LAUNCH(e, launch_rmsnorm_bwd(m->dn, s.x1, L.norm2, d_out, m->dx1, T, H, c.rms_eps, e->stream));
     // B. attention: o projection, attention, RoPE, q | k | v -> dNorm1X; RMSNorm1 backward + residual
     const float *dy_o = m->dx1;
-    rc = backward_group_device(e, 1, L.w + kO, L.ad + kO, &dy_o, s.attn, m->dattn, T, flags);
+    rc = backward_group_device(e, 1, L.w + kO, L.ad + kO, &dy_o, s.attn, m->dattn, T, flags, i16.o ? s.attn16 : nullptr);
     if (rc != GT_OK) return rc;
     rc = attention_backward16_on_device(e, m->dattn, s.q16, s.k16, s.v16, s.attn, s.lse, m->dq, m->dk, m->dv, T, c.n_heads, c.n_kv_heads, c.head_dim);
     if (rc != GT_OK) return rc;
     GT_LAUNCH(e, launch_rope(m->dq, m->dk, T, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_theta, 1.0f, c.head_dim, 1, e->stream));
     const float *dqkv[3] = {m->dq, m->dk, m->dv};
-    rc = backward_group_device(e, 3, L.w + kQ, L.ad + kQ, dqkv, s.n1, m->dn, T, flags);
+    rc = backward_group_device(e, 3, L.w + kQ, L.ad + kQ, dqkv, s.n1, m->dn, T, flags, i16.qkv ? s.n1 : nullptr);
     if (rc != GT_OK) return rc;
     GT_LAUNCH(e, launch_rmsnorm_bwd(m->dn, x_in, L.norm1, m->dx1, d_in, T, H, c.rms_eps, e->stream));
     return GT_OK;
@@ -171,9 +189,22 @@ int stage_inputs(gt_model *m, const int32_t *tokens, const int32_t *labels, int 
 
 int forward_all(gt_model *m, int T, bool keep_states) {
     gt_engine *e = m->eng;
-    int rc = embedding_on_device(e, m->embedding, m->tokens, T, m->x[0], m->bad);
-    if (rc != GT_OK) return rc;
     const int L = (int)m->layers.size();
+    // every adapter's low and dLow of the pass, cleared in a launch or two instead of a few per block
+    std::vector<gt_adapter *> lows;
+    for (int l = 0; l < L; l++)
+        if (inputs16(m, l, T).qkv)
+            for (gt_adapter *a : m->layers[l].ad)
+                if (a && a->rank > 0 && a->scaling != 0.f) lows.push_back(a);
+    struct Forget {      // what the pass did not use is not taken for zeroed later
+        std::vector<gt_adapter *> &v;
+        ~Forget() {
+            for (gt_adapter *a : v) a->zeroed_T = 0;
+        }
+    } forget{lows};
+    int rc = lows.empty() ? GT_OK : clear_lows(e, lows.data(), (int)lows.size(), T);
+    if (rc == GT_OK) rc = embedding_on_device(e, m->embedding, m->tokens, T, m->x[0], m->bad);
+    if (rc != GT_OK) return rc;
     for (int l = 0; l < L; l++) {
         BlockState &s = m->st[keep_states ? l : 0];
         // the norm that follows this block's output rides on its last residual add: the next block's attention norm
@@ -238,7 +269,7 @@ int gt_model_create(gt_engine *e, const gt_model_config *cfg, gt_model **out) {
     const int n_state = c.checkpoint ? 1 : c.n_layers;
     const size_t bh = a256(T * H * 4), bf = a256(T * F * 4), bq = a256(T * QD * 4), bk = a256(T * KD * 4), bl = a256((size_t)c.n_heads * T * 4);
     const size_t bq16 = a256(T * QD * 2), bk16 = a256(T * KD * 2);
-    const size_t state_bytes = 3 * bh + bq + bq16 + 2 * bk16 + bl + 3 * bf;       // n1, x1, n2 | attn | q16 | k16, v16 | lse | gate, up, hidden
+    const size_t state_bytes = 3 * bh + bq + 2 * bq16 + 2 * bk16 + bl + 3 * bf;   // n1, x1, n2 | attn | q16, attn16 | k16, v16 | lse | gate, up, hidden
     size_t total = (size_t)(c.n_layers + 1) * bh + (size_t)n_state * state_bytes + 7 * bh /* tmp, fnorm, dfnorm, dx_a, dx_b, dn, dx1 */ +
                    3 * bq /* q, dattn, dq */ + 4 * bk /* k, v, dk, dv */ + 2 * a256(T * 4) + 1024;
     cudaError_t ce = cudaMalloc((void **)&m->arena, total);
@@ -259,7 +290,7 @@ int gt_model_create(gt_engine *e, const gt_model_config *cfg, gt_model **out) {
     for (BlockState &s : m->st) {
         s.n1 = take(bh); s.x1 = take(bh); s.n2 = take(bh);
         s.attn = take(bq);
-        s.q16 = take(bq16); s.k16 = take(bk16); s.v16 = take(bk16);
+        s.q16 = take(bq16); s.attn16 = take(bq16); s.k16 = take(bk16); s.v16 = take(bk16);
         s.lse = take(bl);
         s.gate = take(bf); s.up = take(bf); s.hidden = take(bf);
     }
