@@ -162,7 +162,7 @@ int compute_low(gt_engine *e, gt_adapter *const *ads, int n, const float *Xd, vo
     if (e->math_mode == GT_MATH_BF16) {
         GT_LAUNCH(e, launch_lora_xa_group(Xd, jobs, n, x16, K, fp16, T, K, fills, n_fills, e->stream));      // fills ride along
     } else {
-        for (int j = 0; j < n_fills; j++) GT_LAUNCH(e, launch_fill_rows(fills[j].dst, fills[j].bias, T, fills[j].N, e->stream));
+        if (n_fills) GT_LAUNCH(e, launch_fill_group(fills, n_fills, T, e->stream));
         for (int j = 0; j < n; j++)
             GT_LAUNCH(e, launch_lora_low(Xd, jobs[j].A, jobs[j].low_zeroed, j == 0 ? x16 : nullptr, K, fp16, T, K, jobs[j].R, e->stream));
     }
@@ -179,8 +179,8 @@ int compute_low16(gt_engine *e, gt_adapter *const *ads, int n, const void *X16, 
     int rc = zero_low(e, ads, n, T);
     if (rc != GT_OK) return rc;
     for (int j = 0; j < n; j++) jobs[j] = LoraXaJob{ads[j]->A, low_of(ads[j]), ads[j]->rank};
-    for (int j = 0; j < n_fills; j++) GT_LAUNCH(e, launch_fill_rows(fills[j].dst, fills[j].bias, T, fills[j].N, e->stream));
-    if (n) GT_LAUNCH(e, launch_lora_xa16_group(X16, K, jobs, n, T, K, e->stream));
+    if (n) GT_LAUNCH(e, launch_lora_xa16_group(X16, K, jobs, n, T, K, fills, n_fills, e->stream));      // fills ride along
+    else if (n_fills) GT_LAUNCH(e, launch_fill_group(fills, n_fills, T, e->stream));
     return GT_OK;
 }
 
@@ -349,7 +349,7 @@ int forward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adap
             if (lora[j]) m[j].lora_act = low_of(ad[j]);       // the adapter's scratch is allocated by now
     } else {
         GT_LAUNCH(e, launch_cast16(Xd, e->x16.p, T, K, K, fp16, e->stream));
-        for (int j = 0; j < n_fills; j++) GT_LAUNCH(e, launch_fill_rows(fills[j].dst, fills[j].bias, T, fills[j].N, e->stream));
+        if (n_fills) GT_LAUNCH(e, launch_fill_group(fills, n_fills, T, e->stream));
     }
     // A Q4_K_M mix gives two launches (q, k in Q4_K | v in Q6_K) that read the same X and write different outputs: the
     // second one runs on the side stream beside the first (neither fills the GPU by itself)
@@ -469,7 +469,7 @@ int lora_backward_group(gt_engine *e, int n, const gt_weight *const *w, gt_adapt
     }
     // "dX =" instead of "dX +=": the buffer is cleared by the pass over dY (or by a fill of its own)
     const RowFill zero{zero_dx, nullptr, K};
-    if (zero_dx && !(fast && nl)) GT_LAUNCH(e, launch_fill_rows(zero_dx, nullptr, T, K, e->stream));
+    if (zero_dx && !(fast && nl)) GT_LAUNCH(e, launch_fill_group(&zero, 1, T, e->stream));
     if (!nl) return GT_OK;
     if (fast) {
         GT_LAUNCH(e, launch_lora_dy_group(dy, nl, fp16, T, zero_dx ? &zero : nullptr, zero_dx ? 1 : 0, e->stream));

@@ -127,20 +127,6 @@ cudaError_t launch_clear(const ClearBuf *bufs, int n, cudaStream_t s) {
     return cudaSuccess;
 }
 
-__global__ void k_fill_rows(float *__restrict__ Y, const float *__restrict__ bias, int T, int N) {
-    pdl_wait();
-    pdl_trigger();
-    const int64_t total = (int64_t)T * N;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
-        Y[i] = bias ? bias[i % N] : 0.f;
-}
-cudaError_t launch_fill_rows(float *Y, const float *bias, int T, int N, cudaStream_t s) {
-    const int64_t total = (int64_t)T * N;
-    if (total <= 0) return cudaSuccess;
-    const unsigned blocks = (unsigned)((total + 255) / 256 > 148 * 8 ? 148 * 8 : (total + 255) / 256);
-    return launch_k(k_fill_rows, dim3(blocks), dim3(256), 0, s, Y, bias, T, N);
-}
-
 __global__ void k_add_inplace(float *__restrict__ dst, const float *__restrict__ src, int64_t n) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) dst[i] += src[i];
 }

@@ -92,8 +92,6 @@ cudaError_t launch_lora_bwd_x(const float *X, const float *dLow, float *dA, floa
 cudaError_t launch_lora_dx_fp32(const float *dLow, const float *A, float *dX, float scaling, int T, int K, int R,
                                 cudaStream_t s);
 cudaError_t launch_cast16(const float *src, void *dst, int rows, int cols, int ld_dst, int fp16, cudaStream_t s);
-// Y[t, :] = bias (or 0)
-cudaError_t launch_fill_rows(float *Y, const float *bias, int T, int N, cudaStream_t s);
 // residual += Y
 cudaError_t launch_add_inplace(float *dst, const float *src, int64_t n, cudaStream_t s);
 // *flag = any(B != 0)
@@ -135,7 +133,10 @@ struct RowFill {
 cudaError_t launch_lora_xa_group(const float *X, const LoraXaJob *jobs, int n, void *x16, int ldx16, int fp16, int T, int K,
                                  const RowFill *fills, int n_fills, cudaStream_t s);
 // the same from an input that already exists as bf16 [T, ld16] (K % 8 == 0, 16-byte aligned): no copy is written
-cudaError_t launch_lora_xa16_group(const void *X16, int ld16, const LoraXaJob *jobs, int n, int T, int K, cudaStream_t s);
+cudaError_t launch_lora_xa16_group(const void *X16, int ld16, const LoraXaJob *jobs, int n, int T, int K, const RowFill *fills, int n_fills,
+                                   cudaStream_t s);
+// the fills alone
+cudaError_t launch_fill_group(const RowFill *fills, int n, int T, cudaStream_t s);
 cudaError_t launch_lora_dy_group(const LoraDyJob *jobs, int n, int fp16, int T, const RowFill *fills, int n_fills, cudaStream_t s);
 // dA from an X that exists as bf16 [T, ld16] (K % 8 == 0, 16-byte aligned)
 cudaError_t launch_lora_da16_group(const void *X16, int ld16, const LoraDaJob *jobs, int n, int T, int K, cudaStream_t s);

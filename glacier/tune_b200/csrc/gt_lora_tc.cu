@@ -88,7 +88,7 @@ struct FillList {
 __device__ __forceinline__ void do_fills(const FillList &fl, int lb, int nb, int tid) {
     for (int j = 0; j < fl.n; j++) {
         const FillList::Job f = fl.f[j];
-        if ((f.N & 3) == 0) {
+        if ((f.N & 3) == 0 && ((reinterpret_cast<uintptr_t>(f.dst) | reinterpret_cast<uintptr_t>(f.bias)) & 15) == 0) {
             const int n4 = f.N >> 2;
             const int64_t total4 = f.total >> 2;
             float4 *d4 = reinterpret_cast<float4 *>(f.dst);
@@ -361,6 +361,7 @@ struct Xa16Params {
     const uint16_t *X16;
     int ld, T, K, n, strips_per_block;
     XaChunk c[kMaxChunks];
+    FillList fills;
 };
 __global__ void __launch_bounds__(256, 2) k_lora_xa16_tc(const Xa16Params p) {
     extern __shared__ __align__(16) uint8_t dyn_smem[];
@@ -438,6 +439,7 @@ __global__ void __launch_bounds__(256, 2) k_lora_xa16_tc(const Xa16Params p) {
 #pragma unroll
         for (int i = 0; i < 2; i++) frag_atomic_add(c.low + c.r0, c.R, d[j][i], t0 + m0 + g, T, i * 8 + 2 * t4, rc, 1.f);
     }
+    do_fills(p.fills, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, tid);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -799,10 +801,30 @@ cudaError_t allow_dyn_smem() {
 
 }  // namespace
 
+__global__ void __launch_bounds__(256) k_fill_group(const FillList fills) {
+    pdl_wait();
+    pdl_trigger();
+    do_fills(fills, blockIdx.x, gridDim.x, threadIdx.x);
+}
+
 static void set_fills(FillList &fl, const RowFill *fills, int n_fills, int T) {
     fl.n = 0;
     for (int j = 0; j < n_fills && fl.n < kMaxChunks; j++)
         fl.f[fl.n++] = FillList::Job{fills[j].dst, fills[j].bias, fills[j].N, (int64_t)T * fills[j].N};
+}
+
+cudaError_t launch_fill_group(const RowFill *fills, int n, int T, cudaStream_t s) {
+    for (int i0 = 0; i0 < n; i0 += kMaxChunks) {
+        FillList fl{};
+        set_fills(fl, fills + i0, n - i0, T);
+        int64_t most = 0;
+        for (int j = 0; j < fl.n; j++) most = fl.f[j].total > most ? fl.f[j].total : most;
+        if (most <= 0) continue;
+        const int64_t want = (most + 4095) / 4096;      // four 16-byte stores per thread and member, 1184 blocks (8 per SM) at most
+        cudaError_t e = launch_k(k_fill_group, dim3((unsigned)(want > 1184 ? 1184 : want)), dim3(256), (size_t)0, s, fl);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_lora_xa_group(const float *X, const LoraXaJob *jobs, int n, void *x16, int ldx16, int fp16, int T, int K,
@@ -838,7 +860,8 @@ cudaError_t launch_lora_xa_group(const float *X, const LoraXaJob *jobs, int n, v
     return flush();
 }
 
-cudaError_t launch_lora_xa16_group(const void *X16, int ld16, const LoraXaJob *jobs, int n, int T, int K, cudaStream_t s) {
+cudaError_t launch_lora_xa16_group(const void *X16, int ld16, const LoraXaJob *jobs, int n, int T, int K, const RowFill *fills, int n_fills,
+                                   cudaStream_t s) {
     if (T <= 0 || K <= 0 || n <= 0) return cudaSuccess;
     if ((K & 7) != 0 || (ld16 & 7) != 0 || (reinterpret_cast<uintptr_t>(X16) & 15) != 0) return cudaErrorInvalidValue;
     static PerDeviceOnce configured;
@@ -854,10 +877,12 @@ cudaError_t launch_lora_xa16_group(const void *X16, int ld16, const LoraXaJob *j
     p.K = K;
     p.strips_per_block = pick_strip_run(strips, 1, T);
     dim3 grid((T + TT - 1) / TT, (strips + p.strips_per_block - 1) / p.strips_per_block);
+    set_fills(p.fills, fills, n_fills, T);      // carried by the first launch
     auto flush = [&]() -> cudaError_t {
         if (p.n == 0) return cudaSuccess;
         cudaError_t le = launch_k(k_lora_xa16_tc, grid, dim3(256), (size_t)(kXsBytes + p.n * kAsBytes), s, p);
         p.n = 0;
+        p.fills.n = 0;
         return le;
     };
     for (int j = 0; j < n; j++)

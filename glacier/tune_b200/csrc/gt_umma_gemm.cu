@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
         }
         for (int i = 0; i < kNumA; i++) {
             // full: the (leader's) producer arrival carrying the TMA bytes + one arrival per dequant warp (of both CTAs)
-            // (a dequant warp counts four times: one group of 4 warps produces a stage, rank-update stages included)
+            // (a dequant warp of the group that decodes a main stage counts four times; all sixteen build a rank-update stage)
             // (fp16 weights: the activation producer and the weight producer, one arrival each)
             mbar_init(bar(kBarFull + i), kDirect ? 2 : 1 + (PAIR ? 32 : 16));
             mbar_init(bar(kBarEmpty + i), 1);                    // tcgen05.commit of the stage's MMAs
@@ -613,116 +613,116 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
             }
         }
         pdl_wait();      // from here on: the low-rank activations, the bias, the output
-        // A rank-update stage is built by the group that owns its slot (n % 4), like any other stage of that slot: the
-        // group has seen every phase of the slot's barriers.  (A group that never waited on a slot could take a phase
-        // two behind for the one it wants - parity waits cannot tell them apart - and the two MMA issuers may be many
-        // stages apart when they run side by side.)
-        for (int lj = 0; lj < n_lora && ok; lj++) {
-            // weight-side tile from B (forward) / A (backward), activation-side tile from the fp32 low-rank activations,
-            // both rounded to T16 here
+        // Rank-update stages: the weight-side tile from B (forward) / A (backward), the activation-side tile from the fp32
+        // low-rank activations, both rounded to T16 here.  Sixteen warps build a stage, 8 ranks of a row per thread and step, and
+        // the first step's loads are in flight before the stage's slot is free: the stage is the last link of the chain, so
+        // every dependent load round trip in it is added to the kernel (by one group of four warps, with 4-byte loads, row by
+        // row: 8 k clocks at 200 tokens and rank 16, of 17 k for a [2816, 1024] projection; now 2.5 k of 9 k).
+        // The group that owns the slot (n % 4) waits for it and the others meet it at a named barrier: only the owner has seen
+        // every phase of the slot's barriers.  (A group that never waited on a slot could take a phase two behind for the one it
+        // wants - parity waits cannot tell them apart - and the two MMA issuers may be many stages apart when they run side by
+        // side.)  All sixteen warps come to the barrier, also those whose own wait gave up (the abort flag is set then).
+        for (int lj = 0; lj < n_lora; lj++) {
+            const bool dual = !BWD && p.dual;
             const Member &L = p.m[lora_m[lj]];
-            const int rank_pad = (!BWD && p.dual) ? dual_pad[0] + dual_pad[1] : (L.rank + 15) & ~15;
+            const int rank_pad = dual ? dual_pad[0] + dual_pad[1] : (L.rank + 15) & ~15;
+            const int nch = rank_pad >> 3;      // 16-byte chunks of an operand row
             const int n = sub * nu + lj;
             const int ai = n % kNumA;
-            if (ai != g4) continue;
-            ok = mbar_wait_bounded(bar(kBarEmpty + ai), ((uint32_t)(n / kNumA) & 1u) ^ 1u, abort_flag, p.status, kCodeDequant + 3);
-            if (!ok) break;
-            const uint32_t a_addr = sbase + kOffA + ai * kAStageBytes;
-            if (!BWD && p.dual) {
-                // one stage for both members: contraction columns [0, pad0) are member 0's ranks, [pad0, pad0 + pad1) member
-                // 1's; a member's weight-side rows are zero in the other member's columns
-                const uint32_t x_addr = sbase + kOffX + ai * kXStageBytes;
-                for (int i = 0; i < n_mma; i++) {
-                    const int ntok = min(MTOK, tb - MTOK * i);
-                    const int rows = PAIR ? (ntok >> 1) : ntok;
-                    for (int rr = dt; rr < rows; rr += 128) {
-                        const int t = tok0 + MTOK * i + (PAIR ? (int)crank * rows : 0) + rr;
-                        const uint32_t row_addr = x_addr + (uint32_t)(i * kMmaSlotBytes + rr * 128);
-                        for (int j = 0; j * 8 < rank_pad; j++) {
-                            const int mm = 8 * j < dual_pad[0] ? 0 : 1;
-                            const Member &Lm = p.m[mm];
-                            const int rbase = 8 * j - (mm ? dual_pad[0] : 0);
-                            float v[8];
+            const int st = threadIdx.x - 64;    // 0 .. 511
+            auto ld8 = [](const float *src, int valid, float (&v)[8]) {
+                if (valid >= 8 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+                    const float4 x = *reinterpret_cast<const float4 *>(src), y = *reinterpret_cast<const float4 *>(src + 4);
+                    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+                } else {
 #pragma unroll
-                            for (int q = 0; q < 8; q++) {
-                                const int r = rbase + q;
-                                v[q] = (r < Lm.rank && t < p.T) ? Lm.lora_act[(int64_t)t * Lm.rank + r] * Lm.lora_scale : 0.f;
-                            }
-                            st_shared_v4(row_addr + (uint32_t)((j ^ (rr & 7)) << 4), pack2<T16>(v[0], v[1]), pack2<T16>(v[2], v[3]),
-                                         pack2<T16>(v[4], v[5]), pack2<T16>(v[6], v[7]));
-                        }
-                    }
+                    for (int q = 0; q < 8; q++) v[q] = q < valid ? src[q] : 0.f;
                 }
-                {
-                    const int row = dt, mm = row >> 6, nn = ltile * 64 + (row & 63), prow = dual_row(row);
-                    const Member &Lm = p.m[mm];
-                    for (int j = 0; j * 8 < rank_pad; j++) {
-                        const bool mine = (8 * j < dual_pad[0]) == (mm == 0) && dual_pad[mm] > 0;
-                        const int rbase = 8 * j - (mm ? dual_pad[0] : 0);
-                        float v[8];
+            };
+            // chunk j of a stage: member and first rank.  Dual: one stage for both members - contraction columns [0, pad0) are member
+            // 0's ranks, [pad0, pad0 + pad1) member 1's; a member's weight-side rows are zero in the other member's columns
+            auto chunk = [&](int j, int &r0) -> int {
+                const int mm = dual && 8 * j >= dual_pad[0] ? 1 : 0;
+                r0 = 8 * j - (mm ? dual_pad[0] : 0);
+                return dual ? mm : lora_m[lj];
+            };
+            // activation side: item = (token row of this CTA's tile, chunk), the chunks of a row beside each other
+            constexpr int kRowsPerMma = PAIR ? MTOK / 2 : MTOK;
+            const int x_items = (PAIR ? tb >> 1 : tb) * nch;
+            auto x_load = [&](int it, float (&v)[8]) {
+                const int ridx = it / nch, i = ridx / kRowsPerMma, rr = ridx % kRowsPerMma;
+                const int half = min(MTOK, tb - MTOK * i) >> 1;
+                const int t = tok0 + MTOK * i + (PAIR ? (int)crank * half : 0) + rr;
+                int r0;
+                const Member &Lm = p.m[chunk(it % nch, r0)];
+                ld8(Lm.lora_act + (int64_t)t * Lm.rank + r0, t < p.T ? Lm.rank - r0 : 0, v);
 #pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const int r = rbase + i;
-                            v[i] = (mine && r < Lm.rank && nn < Lm.N) ? Lm.lora_w[(int64_t)r * Lm.N + nn] : 0.f;
-                        }
-                        st_shared_v4(a_addr + (uint32_t)(prow * 128 + ((j ^ (prow & 7)) << 4)), pack2<T16>(v[0], v[1]),
-                                     pack2<T16>(v[2], v[3]), pack2<T16>(v[4], v[5]), pack2<T16>(v[6], v[7]));
-                    }
+                for (int q = 0; q < 8; q++) v[q] *= Lm.lora_scale;
+            };
+            auto x_store = [&](int it, const float (&v)[8]) {
+                const int ridx = it / nch, i = ridx / kRowsPerMma, rr = ridx % kRowsPerMma, j = it % nch;
+                st_shared_v4(sbase + kOffX + ai * kXStageBytes + (uint32_t)(i * kMmaSlotBytes + rr * 128 + ((j ^ (rr & 7)) << 4)),
+                             pack2<T16>(v[0], v[1]), pack2<T16>(v[2], v[3]), pack2<T16>(v[4], v[5]), pack2<T16>(v[6], v[7]));
+            };
+            // weight side: item = (chunk, row or column of the tile)
+            const int w_items = 128 * nch;
+            auto w_load = [&](int it, float (&v)[8]) {
+                const int row = it & 127;
+                int r0;
+                const int mj = chunk(it >> 7, r0);
+                const Member &Lm = p.m[mj];
+                if (BWD) {
+                    const int k = tile * kTileW + row;
+                    ld8(Lm.lora_w + (int64_t)k * Lm.rank + r0, k < p.K ? Lm.rank - r0 : 0, v);
+                } else {
+                    const int nn = dual ? ltile * 64 + (row & 63) : ltile * kTileW + row;
+                    const bool mine = nn < Lm.N && (!dual || (row >> 6) == mj);
+#pragma unroll
+                    for (int q = 0; q < 8; q++) v[q] = mine && r0 + q < Lm.rank ? Lm.lora_w[(int64_t)(r0 + q) * Lm.N + nn] : 0.f;
                 }
-                fence_proxy_async_smem();
-                __syncwarp();
-                signal_a_full(ai, 4);
-                continue;
+            };
+            auto w_store = [&](int it, const float (&v)[8]) {
+                const int row = it & 127, j = it >> 7;
+                const uint32_t a_addr = sbase + kOffA + ai * kAStageBytes;
+                if (BWD) {      // image(col >> 6)[row = r][col & 63] = A[k, r]
+                    const int c = row & 63;
+#pragma unroll
+                    for (int q = 0; q < 8; q++) {
+                        const uint32_t bits = pack2<T16>(v[q], 0.f) & 0xFFFFu;
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(a_addr + (uint32_t)((row >> 6) * 8192 + (8 * j + q) * 128 +
+                                                                                        (((c >> 3) ^ q) << 4) + (c & 7) * 2)),
+                                     "h"((unsigned short)bits)
+                                     : "memory");
+                    }
+                } else {        // image[row = n][col = r] = B[r, n]
+                    const int prow = dual ? dual_row(row) : row;
+                    st_shared_v4(a_addr + (uint32_t)(prow * 128 + ((j ^ (prow & 7)) << 4)), pack2<T16>(v[0], v[1]), pack2<T16>(v[2], v[3]),
+                                 pack2<T16>(v[4], v[5]), pack2<T16>(v[6], v[7]));
+                }
+            };
+            float xv[8], wv[8];
+            if (st < x_items) x_load(st, xv);
+            if (st < w_items) w_load(st, wv);
+            if (ok && (n & 3) == g4)
+                ok = mbar_wait_bounded(bar(kBarEmpty + ai), ((uint32_t)(n / kNumA) & 1u) ^ 1u, abort_flag, p.status, kCodeDequant + 3);
+            asm volatile("bar.sync 5, 512;" ::: "memory");
+            if (*abort_flag) ok = false;
+            if (!ok) continue;
+            if (st < x_items) x_store(st, xv);
+            if (st < w_items) w_store(st, wv);
+#pragma unroll 1
+            for (int it = st + 512; it < x_items; it += 512) {
+                x_load(it, xv);
+                x_store(it, xv);
             }
-            {
-                // token rows of this CTA's activation tile: rank_pad/8 chunks of a 128-byte row
-                const uint32_t x_addr = sbase + kOffX + ai * kXStageBytes;
-                for (int i = 0; i < n_mma; i++) {
-                    const int ntok = min(MTOK, tb - MTOK * i);
-                    const int rows = PAIR ? (ntok >> 1) : ntok;
-                    for (int rr = dt; rr < rows; rr += 128) {
-                        const int t = tok0 + MTOK * i + (PAIR ? (int)crank * rows : 0) + rr;
-                        const uint32_t row_addr = x_addr + (uint32_t)(i * kMmaSlotBytes + rr * 128);
-                        for (int j = 0; j * 8 < rank_pad; j++) {
-                            float v[8];
-#pragma unroll
-                            for (int q = 0; q < 8; q++) {
-                                const int r = 8 * j + q;
-                                v[q] = (r < L.rank && t < p.T) ? L.lora_act[(int64_t)t * L.rank + r] * L.lora_scale : 0.f;
-                            }
-                            st_shared_v4(row_addr + (uint32_t)((j ^ (rr & 7)) << 4), pack2<T16>(v[0], v[1]), pack2<T16>(v[2], v[3]),
-                                         pack2<T16>(v[4], v[5]), pack2<T16>(v[6], v[7]));
-                        }
-                    }
-                }
-            }
-            if (!BWD) {
-                // image[row = n][col = r] = B[r, n]; chunks of 8 ranks
-                const int row = dt, nn = ltile * kTileW + row;
-                for (int j = 0; j * 8 < rank_pad; j++) {
-                    float v[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const int r = 8 * j + i;
-                        v[i] = (r < L.rank && nn < L.N) ? L.lora_w[(int64_t)r * L.N + nn] : 0.f;
-                    }
-                    st_shared_v4(a_addr + (uint32_t)(row * 128 + ((j ^ (row & 7)) << 4)), pack2<T16>(v[0], v[1]),
-                                 pack2<T16>(v[2], v[3]), pack2<T16>(v[4], v[5]), pack2<T16>(v[6], v[7]));
-                }
-            } else {
-                // image(kcol >> 6)[row = r][col = kcol & 63] = A[k, r]
-                const int kcol = dt, c = kcol & 63, k = tile * kTileW + kcol;
-                for (int r = 0; r < rank_pad; r++) {
-                    const float v = (r < L.rank && k < p.K) ? L.lora_w[(int64_t)k * L.rank + r] : 0.f;
-                    const uint32_t addr =
-                        a_addr + (uint32_t)((kcol >> 6) * 8192 + r * 128 + (((c >> 3) ^ (r & 7)) << 4) + (c & 7) * 2);
-                    const uint32_t bits = pack2<T16>(v, 0.f) & 0xFFFFu;
-                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"((unsigned short)bits) : "memory");
-                }
+#pragma unroll 1
+            for (int it = st + 512; it < w_items; it += 512) {
+                w_load(it, wv);
+                w_store(it, wv);
             }
             fence_proxy_async_smem();
             __syncwarp();
-            signal_a_full(ai, 4);
+            signal_a_full(ai, 1);
         }
         // epilogue: TMEM lane = weight row / column of this tile, TMEM column = token
         if (ok) ok = mbar_wait_bounded(bar(kBarAcc), 0u, abort_flag, p.status, kCodeEpilogue + 1, 16000000000ll);
