@@ -170,11 +170,12 @@ int compute_low(gt_engine *e, gt_adapter *const *ads, int n, const float *Xd, vo
 }
 
 // The same from an X that already exists as bf16 [T, K] (bf16 mode only): low_j = X16 * A_j, no copy is written.
-// keep: a low_j of this T that is in place stays.
+// keep: a low_j of this T that is in place stays.  *launched (may be null): a kernel went out.
 int compute_low16(gt_engine *e, gt_adapter *const *ads, int n, const void *X16, int T, int K, const RowFill *fills = nullptr,
-                  int n_fills = 0, bool keep = false) {
+                  int n_fills = 0, bool keep = false, int *launched = nullptr) {
     for (int j = 0; j < n; j++) keep = keep && ads[j]->low.p && ads[j]->low_T == T;
     if (keep) n = 0;
+    if (launched) *launched = n || n_fills ? 1 : 0;
     LoraXaJob jobs[kMaxGroup];
     int rc = zero_low(e, ads, n, T);
     if (rc != GT_OK) return rc;
@@ -323,11 +324,12 @@ int forward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adap
     int n_fills = 0;
     for (int r = 0, pos = 0; r < runs; pos += count[r], r++) {
         for (int i = 0; i < count[r]; i++) run_m[pos + i] = m[order[pos + i]];
-        const int splits = dual_h16 ? 1 : umma_group_splits(run_m + pos, count[r], e->sm_count);
+        umma_group_plan(run_m + pos, count[r], e->sm_count, dual_h16 != nullptr);
         for (int i = 0; i < count[r]; i++) {
             const int j = order[pos + i];
-            m[j].splits = splits;
-            if (splits > 1) {
+            m[j].splits = run_m[pos + i].splits;
+            m[j].tok_chunk = run_m[pos + i].tok_chunk;
+            if (m[j].splits > 1) {
                 fills[n_fills++] = RowFill{Yd[j], w[j]->dev.bias, w[j]->dev.N};
                 m[j].out_prefilled = 1;
             }
@@ -338,10 +340,13 @@ int forward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adap
     for (int j = 0; j < n; j++)
         if (lora[j]) with[n_with++] = ad[j];
     if (x16_ready) {
-        int rc = compute_low16(e, with, n_with, x16_ready, T, K, fills, n_fills, (flags & kFlagKeepLow) != 0);
+        int early = 0;
+        int rc = compute_low16(e, with, n_with, x16_ready, T, K, fills, n_fills, (flags & kFlagKeepLow) != 0, &early);
         if (rc != GT_OK) return rc;
-        for (int j = 0; j < n; j++)
+        for (int j = 0; j < n; j++) {
             if (lora[j]) m[j].lora_act = low_of(ad[j]);
+            m[j].act_early = early;
+        }
     } else if (n_with) {
         int rc = compute_low(e, with, n_with, Xd, e->x16.p, fp16, T, K, fills, n_fills);
         if (rc != GT_OK) return rc;
@@ -549,14 +554,18 @@ int backward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_ada
     // one launch per quantization type, all summing into the same dX.  "dX =": when the first launch has one CTA per
     // output tile (no split-K) it writes dX with plain stores and nothing has to clear the buffer first; otherwise the
     // pass over dY (or a fill of its own) clears it and every launch adds.
-    int order[kMaxGroup], count[kMaxGroup], run_splits[kMaxGroup];
+    int order[kMaxGroup], count[kMaxGroup];
     const int runs = partition_by_type(n, w, order, count);
     UmmaLaunch run_m[kMaxGroup];
     for (int r = 0, pos = 0; r < runs; pos += count[r], r++) {
         for (int i = 0; i < count[r]; i++) run_m[pos + i] = m[order[pos + i]];
-        run_splits[r] = umma_group_splits(run_m + pos, count[r], e->sm_count);
+        umma_group_plan(run_m + pos, count[r], e->sm_count);
+        for (int i = 0; i < count[r]; i++) {
+            m[order[pos + i]].splits = run_m[pos + i].splits;
+            m[order[pos + i]].tok_chunk = run_m[pos + i].tok_chunk;
+        }
     }
-    const bool store_first = assign && run_splits[0] == 1;
+    const bool store_first = assign && run_m[0].splits == 1;
     int rc = lora_backward_group(e, n, w, ad, lora, dYd, Xd, dy16, ld16, T, reuse_low, (assign && !store_first) ? dXd : nullptr,
                                  side_da_enabled() && !e->profile,       // profiling times each GEMM alone on the device
                                  e->math_mode == GT_MATH_BF16 ? X16 : nullptr);
@@ -567,6 +576,8 @@ int backward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_ada
             m[j].lora_scale = ad[j]->scaling;
             m[j].lora_w = ad[j]->A;
             m[j].rank = ad[j]->rank;
+            if (dy16_ready)      // the pass over dY came after whatever wrote its 16-bit copy
+                for (int i = 0; i < n; i++) m[i].act_early = 1;
         }
     }
     // A run served by the few-token kernel adds its adapter terms to dX with plain read-modify-writes: then no run of
@@ -577,10 +588,7 @@ int backward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_ada
         any_few = any_few || umma_group_few(run_m + pos, count[r]);
     }
     for (int r = 0, pos = 0; r < runs; pos += count[r], r++) {
-        for (int i = 0; i < count[r]; i++) {
-            run_m[pos + i] = m[order[pos + i]];
-            run_m[pos + i].splits = run_splits[r];
-        }
+        for (int i = 0; i < count[r]; i++) run_m[pos + i] = m[order[pos + i]];
         run_m[pos].out_assign = (r == 0 && store_first) ? 1 : 0;
         // launches of the other quantization types add into the same dX with atomics: beside the first one on the side
         // stream (behind the dA pass there), unless the first one writes dX with plain stores

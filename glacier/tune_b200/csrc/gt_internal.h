@@ -149,6 +149,8 @@ struct UmmaLaunch {
     int fp16 = 0;                  // operand format: 0 bf16, 1 fp16
     const void *act16 = nullptr;   // 16-bit activations [T, ld_act]
     int ld_act = 0;
+    int act_early = 0;             // member 0: the kernel launched right before does not write act16, and waited for the one that did
+                                   // before it let this one start: the main loop need not wait for it
     int T = 0;
     float *out = nullptr;          // fp32 [T, ld_out]
     int ld_out = 0;
@@ -163,6 +165,7 @@ struct UmmaLaunch {
     int rank = 0;
     const int *lora_flag = nullptr;     // device int: 0 -> skip the update
     int splits = 1;
+    int tok_chunk = 0;                  // tokens per CTA (umma_group_plan); 0: as many as a CTA can take
     int *status = nullptr;              // device int[4]
     void *trace = nullptr;              // optional device int64[12*128] timeline buffer
     // a window of the weight's rows [row_base, row_base + rows) instead of all of them (rows == 0: the whole tensor):
@@ -183,7 +186,7 @@ bool tmap_encode_2d(CUtensorMap *tm, CUtensorMapDataType dt, const void *base, u
                     uint32_t b0, uint32_t b1, CUtensorMapSwizzle swz);
 // Up to three projections in one launch (see gt_umma_gemm.cu); umma_group_ok tells whether they qualify.
 bool umma_group_ok(const UmmaLaunch *m, int n);
-int umma_group_splits(const UmmaLaunch *m, int n, int sm_count);
+void umma_group_plan(UmmaLaunch *m, int n, int sm_count, bool dual = false);      // sets splits and tok_chunk
 // dual forward (gate | up, SwiGLU product in the epilogue): see umma_dual_ok
 struct UmmaDual {
     void *h16 = nullptr;      // 16-bit [T, ld_h16] in the launch's operand format, or null

@@ -322,7 +322,7 @@ UmmaLaunch head_launch(gt_engine *e, const WeightDev *w, bool backward, const vo
     L.rows = rows;
     L.status = e->status;
     L.trace = e->trace;
-    L.splits = umma_group_splits(&L, 1, e->sm_count);
+    umma_group_plan(&L, 1, e->sm_count);
     return L;
 }
 

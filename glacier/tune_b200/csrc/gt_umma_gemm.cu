@@ -116,6 +116,8 @@ struct Params {
     // Rows of an odd number of half super-blocks (in_features % 256 == 128): the byte stream is addressed as rows of two
     // weight rows each (whole super-blocks again); weight row 2 s + h starts pair_hb * h half-blocks into row s.  0: plain rows
     int pair_hb;
+    int act_early;      // see UmmaLaunch
+    int tok_chunk;      // token rows per CTA (grid.z chunks), at most kMaxTok and a multiple of 32
     void *h16;       // T16 [T, ld_h16]: SiLU(gate) * up, or null
     int ld_h16;
 };
@@ -228,10 +230,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
     const int tile = blockIdx.x, split = blockIdx.y;
     const uint32_t crank = PAIR ? cluster_ctarank() : 0u;        // 0 = leader
     const bool leader = crank == 0;
-    const int tok0 = blockIdx.z * kMaxTok;
+    const int tok0 = blockIdx.z * p.tok_chunk;
     const int tok_left = p.T - tok0;
     // token columns of this CTA's accumulator: multiple of 16 (single) / 32 (pair, 16 per CTA half)
-    const int tb = PAIR ? min(kMaxTok, (tok_left + 31) & ~31) : min(kMaxTok, (tok_left + 15) & ~15);
+    const int tb = PAIR ? min(p.tok_chunk, (tok_left + 31) & ~31) : min(p.tok_chunk, (tok_left + 15) & ~15);
     const int n_box = (tb + p.t_box - 1) / p.t_box;             // single-CTA mode: TMA boxes per stage
     const int n_mma = (tb + MTOK - 1) / MTOK;
     // Few tokens (single-CTA mode): the four k-steps of a stage go to separate accumulators, so they do not wait on
@@ -423,7 +425,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_umma_gemm(const __grid_constant
         if (lane < 4) {
             Ring xs;
             bool ok = true;
-            pdl_wait();      // the activations come from the kernel before this one
+            // the activations come from the kernel before this one, or from one that had completed when this one was scheduled
+            // (act_early: 28 blocks of 3584 features, 512 tokens: 26.1 -> 25.8 ms for a training pass)
+            if (!p.act_early) pdl_wait();
             for (int u = u0; u < u1 && ok; u++) {
                 int um = mi, rb = 0;
                 if (BWD) um = unit_member(u, rb);
@@ -948,10 +952,10 @@ cudaError_t launch_one(const Params &p, dim3 grid, bool pair, cudaStream_t s) {
     static const bool deep = !(getenv("GT_DEEP_RING") && atoi(getenv("GT_DEEP_RING")) == 0);
     if (pair) {
         if (p.t_box == 64) return launch_variant<QT, T16, BWD, true, 128, 256>(p, grid, s);
-        if (QT != kTypeF16 && deep && p.T <= 256) return launch_variant<QT, T16, BWD, true, 256, 128>(p, grid, s);
+        if (QT != kTypeF16 && deep && (p.T <= 256 || p.tok_chunk <= 256)) return launch_variant<QT, T16, BWD, true, 256, 128>(p, grid, s);
         return launch_variant<QT, T16, BWD, true, 256, 256>(p, grid, s);
     }
-    if (QT != kTypeF16 && deep && p.T <= 128) return launch_variant<QT, T16, BWD, false, 256, 128>(p, grid, s);
+    if (QT != kTypeF16 && deep && (p.T <= 128 || p.tok_chunk <= 128)) return launch_variant<QT, T16, BWD, false, 256, 128>(p, grid, s);
     return launch_variant<QT, T16, BWD, false, 256, 256>(p, grid, s);
 }
 
@@ -1025,16 +1029,15 @@ static bool half_units(const WeightDev *w, bool pair) { return !pair || w->qtype
 static int fwd_units(const WeightDev *w, bool pair) { return half_units(w, pair) ? w->K / 128 : w->K / 256; }
 
 // at least four (backward: two) 64-deep operand stages per split
-static int pick_splits(int tiles, int max_splits, int T, int sm_count) {
-    const int chunks = (T + kMaxTok - 1) / kMaxTok;
-    int s = sm_count / (tiles * chunks > 0 ? tiles * chunks : 1);
+static int pick_splits(int ctas, int max_splits, int sm_count) {
+    int s = sm_count / (ctas > 0 ? ctas : 1);
     if (s > max_splits) s = max_splits;
     return s < 1 ? 1 : s;
 }
 
 int umma_pick_splits(const WeightDev *w, int backward, int T, int sm_count) {
     const int tiles = backward ? w->K / kTileW : (w->N + kTileW - 1) / kTileW;
-    return pick_splits(tiles, backward ? (w->N + 63) / 64 / 2 : w->K / 256, T, sm_count);
+    return pick_splits(tiles * ((T + kMaxTok - 1) / kMaxTok), backward ? (w->N + 63) / 64 / 2 : w->K / 256, sm_count);
 }
 
 bool umma_group_ok(const UmmaLaunch *m, int n) {
@@ -1052,12 +1055,13 @@ bool umma_group_ok(const UmmaLaunch *m, int n) {
     return true;
 }
 
-// CTA pairs pay off once the activation tile is the bulk of what an SM pulls from L2, and they halve the MMA
-// instructions per weight; pair mode needs 16 token columns per CTA half (the knob is clamped to [32, 256])
+// A CTA takes up to 256 tokens alone (its activation stages hold 256 rows), more as half of a CTA pair: [18944, 3584] in Q4_K, 256
+// tokens: 39 k clocks alone, 59 k as a pair, whose stages go round between two SMs.  The knob is clamped to [32, 257] (pair mode
+// needs 16 token columns per CTA half).
 static int pair_min_tokens() {
     static const int pair_min = [] {
-        const int v = getenv("GT_PAIR_MIN") ? atoi(getenv("GT_PAIR_MIN")) : 256;
-        return v < 32 ? 32 : (v > 256 ? 256 : v);
+        const int v = getenv("GT_PAIR_MIN") ? atoi(getenv("GT_PAIR_MIN")) : 257;
+        return v < 32 ? 32 : (v > 257 ? 257 : v);
     }();
     return pair_min;
 }
@@ -1070,9 +1074,52 @@ static bool few_group(const UmmaLaunch *m, int n) {
 }
 bool umma_group_few(const UmmaLaunch *m, int n) { return few_group(m, n); }
 
-int umma_group_splits(const UmmaLaunch *m, int n, int sm_count) {
+// How a launch is cut: token chunks (grid.z; their size goes into the launches' tok_chunk) and contraction splits.  Every split
+// and every chunk costs a CTA its start, its pipeline fill and the drain of its accumulator; more of them fill the SMs where there
+// are few weight tiles.  The candidates - as few chunks as 512 tokens each allow, and every larger number of them down to 96
+// tokens - are priced with the clocks of the kernel's own time stamps ([18944, 3584], 96 to 512 tokens, both types and
+// directions): 6.5 k to start, 64-deep stages at 600 for a CTA alone (880 for Q6_K from 129 tokens on, where two raw stages
+// are in flight instead of six) and 870 + 0.53 per token in a pair, 700 + 20 per token to drain.  More chunks than needed are
+// taken where they are 3 % cheaper.
+static void pick_plan(UmmaLaunch *m, int n, int sm_count, bool dual) {
     const bool bwd = m[0].backward != 0;
-    if (few_group(m, n)) {
+    const int T = m[0].T;
+    const WeightDev *w0 = m[0].w;
+    const int nc0 = (T + kMaxTok - 1) / kMaxTok;
+    const int nc1 = w0->qtype == kTypeF16 ? nc0 : (T + 95) / 96;      // (fp16 rows: vocabulary tiles, always many)
+    double best = 0.;
+    int splits = 1, chunk = 0;
+    for (int nc = nc0; nc <= nc1; nc++) {
+        const int c = ((T + nc - 1) / nc + 31) & ~31;
+        if ((T + c - 1) / c != nc || c > kMaxTok || (dual && c <= 128 && nc > nc0)) continue;
+        const bool pair = (nc == 1 ? T : c) >= pair_min_tokens();
+        int tiles = 0, stages = bwd ? 0 : w0->K / 64;
+        for (int j = 0; j < n; j++) {
+            const int rows = eff_rows(m[j]);
+            int t = bwd ? w0->K / kTileW : (dual ? (j == 0 ? rows / 64 : 0) : (rows + kTileW - 1) / kTileW);
+            if (pair) t = (t + 1) & ~1;
+            tiles = bwd ? t : tiles + t;
+            if (bwd) stages += (rows + 63) / 64;
+        }
+        const int sp = dual ? 1 : pick_splits(tiles * nc, bwd ? stages / 2 : stages / 4, sm_count);
+        const int waves = (tiles * nc * sp + sm_count - 1) / (sm_count > 0 ? sm_count : 1);
+        const double stage = pair ? 870. + 0.53 * c : (w0->qtype == kTypeQ6K && c > 128 ? 880. : 600.);
+        const double cost = waves * (6500. + (stages + sp - 1) / sp * stage + 700. + 20. * c) + (sp > 1 ? 1500. : 0.);
+        if (chunk == 0 || cost < 0.97 * best) {
+            best = cost;
+            splits = sp;
+            chunk = c;
+        }
+    }
+    for (int j = 0; j < n; j++) {
+        m[j].splits = splits;
+        m[j].tok_chunk = chunk;
+    }
+}
+
+void umma_group_plan(UmmaLaunch *m, int n, int sm_count, bool dual) {
+    const bool bwd = m[0].backward != 0;
+    if (!dual && few_group(m, n)) {
         // one launch per member, all with the same split count: forward sized for the members' tiles together (they run
         // back to back), backward for the longest contraction
         int tiles = 0, units = 0;
@@ -1091,47 +1138,36 @@ int umma_group_splits(const UmmaLaunch *m, int n, int sm_count) {
         int sp = sm_count / (tiles > 0 ? tiles : 1);
         const int cap = bwd ? (units / 2 > 1 ? units / 2 : 1) : units;
         if (sp > cap) sp = cap;
-        return sp < 1 ? 1 : sp;
+        for (int j = 0; j < n; j++) m[j].splits = sp < 1 ? 1 : sp;
+        return;
     }
-    const int tmax = m[0].T < kMaxTok ? m[0].T : kMaxTok;
-    const bool pair = tmax >= pair_min_tokens();
-    int tiles = 0, units = 0;
-    for (int j = 0; j < n; j++) {
-        const WeightDev *w = m[j].w;
-        const int rows = eff_rows(m[j]);
-        if (bwd) {
-            units += (rows + 63) / 64;
-            tiles = w->K / kTileW;
-            if (pair) tiles = (tiles + 1) & ~1;
-        } else {
-            int t = (rows + kTileW - 1) / kTileW;
-            if (pair) t = (t + 1) & ~1;
-            tiles += t;
-            units = w->K / 128;
-        }
-    }
-    return pick_splits(tiles, units / 2, m[0].T, sm_count);
+    pick_plan(m, n, sm_count, dual);
 }
 
 // Members share T, math mode, direction, in_features and quantization type (umma_group_ok).  Forward: the activation
 // operand and `splits` / `out_prefilled` come from member 0.  Backward: every member brings its own dY; `out` is shared.
 // gate | up with the SwiGLU product in the epilogue: members 0 and 1 of the same shape and type, no split-K; either
 // member's `out` may be null (nothing but the product is wanted), h16 receives SiLU(out0) * out1 as 16-bit values
-bool umma_dual_ok(const UmmaLaunch *m, int sm_count) {
+static bool dual_shape_ok(const UmmaLaunch *m) {
     if (!umma_group_ok(m, 2) || m[0].backward || few_group(m, 2)) return false;
     const WeightDev *a = m[0].w, *b = m[1].w;
     if (a->qtype == kTypeF16 || a->pair_hb || a->N != b->N || a->N % 64 != 0 || m[0].rows || m[1].rows) return false;
     if (m[0].rank > 32 || m[1].rank > 32 || m[0].out_prefilled || m[1].out_prefilled) return false;
-    if (m[0].T <= 128) return false;      // the kernel's 256-row activation stages
+    return m[0].T > 128;      // the kernel's 256-row activation stages
+}
+bool umma_dual_ok(const UmmaLaunch *m, int sm_count) {
+    if (!dual_shape_ok(m)) return false;
     // one CTA per 64 features and token chunk, no split-K: worth it where those alone fill the GPU
     // (GT_FFN_DUAL_MIN_TILES, read at every call: a smaller bound, for tests on small tensors)
     const char *env = getenv("GT_FFN_DUAL_MIN_TILES");
     const int need = env ? atoi(env) : sm_count;
-    return (a->N / 64) * ((m[0].T + kMaxTok - 1) / kMaxTok) >= need;
+    UmmaLaunch plan[2] = {m[0], m[1]};
+    pick_plan(plan, 2, sm_count, true);
+    return (m[0].w->N / 64) * ((m[0].T + plan[0].tok_chunk - 1) / plan[0].tok_chunk) >= need;
 }
 
 cudaError_t launch_umma_group(const UmmaLaunch *m, int n, cudaStream_t s, const char **err, const UmmaDual *dual) {
-    if (dual && (n != 2 || !umma_dual_ok(m, 0))) {
+    if (dual && (n != 2 || !dual_shape_ok(m))) {
         if (err) *err = "the two projections do not qualify for the dual forward";
         return cudaErrorInvalidValue;
     }
@@ -1168,7 +1204,8 @@ cudaError_t launch_umma_group(const UmmaLaunch *m, int n, cudaStream_t s, const 
     }
     Params p;
     memset(&p, 0, sizeof(p));
-    const int tmax = L0.T < kMaxTok ? L0.T : kMaxTok;
+    p.tok_chunk = L0.tok_chunk > 0 && L0.tok_chunk < kMaxTok ? L0.tok_chunk : kMaxTok;
+    const int tmax = L0.T < p.tok_chunk ? L0.T : p.tok_chunk;
     const bool pair = tmax >= pair_min_tokens();
     const int tb = pair ? (tmax + 31) & ~31 : (tmax + 15) & ~15;
     // pair mode: TMA box rows = half of an MMA's token columns (64 with four 128-column accumulators)
@@ -1237,6 +1274,7 @@ cudaError_t launch_umma_group(const UmmaLaunch *m, int n, cudaStream_t s, const 
         first += count;
     }
     p.pair_hb = L0.w->pair_hb;
+    p.act_early = L0.act_early;
     p.status = L0.status;
     p.trace = (long long *)L0.trace;
     p.T = L0.T;
@@ -1256,7 +1294,7 @@ cudaError_t launch_umma_group(const UmmaLaunch *m, int n, cudaStream_t s, const 
     // 256 == 128): the padding tile reads zero-filled weights and stores nothing
     int tiles = bwd ? L0.w->K / kTileW : first;
     if (bwd && pair) tiles = (tiles + 1) & ~1;
-    dim3 grid(tiles, p.splits, (L0.T + kMaxTok - 1) / kMaxTok);
+    dim3 grid(tiles, p.splits, (L0.T + p.tok_chunk - 1) / p.tok_chunk);
     const int qt = L0.w->qtype;
     if (qt == kTypeF16) return bwd ? launch_one<kTypeF16, __half, true>(p, grid, pair, s) : launch_one<kTypeF16, __half, false>(p, grid, pair, s);
     if (qt == kTypeQ4K) {
