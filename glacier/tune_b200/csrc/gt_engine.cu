@@ -513,6 +513,13 @@ static size_t dy16_layout(int n, const gt_weight *const *w, int T, size_t *off, 
     return total;
 }
 
+int reserve_dy16(gt_engine *e, int n, const gt_weight *const *w, int T) {
+    size_t off[kMaxGroup];
+    int ld[kMaxGroup];
+    GT_CUDA(e->dy16.reserve(dy16_layout(n, w, T, off, ld)));
+    return GT_OK;
+}
+
 int backward_group_device(gt_engine *e, int n, const gt_weight *const *w, gt_adapter *const *ad, const float *const *dYd,
                           const float *Xd, float *dXd, int T, int flags, const void *X16, bool dy16_ready) {
     bool lora[kMaxGroup];
@@ -757,7 +764,7 @@ int ffn_forward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *cons
 // dX (+)= dGate * W_gate + dUp * W_up (+ adapters); adapter gradients accumulate.  Device tensors.
 int ffn_backward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *const *ad, const float *dYd, const float *Xd,
                         const float *gate_d, const float *up_d, const float *hidden_d, float *dXd, int T, int flags,
-                        const void *hidden16, const void *X16) {
+                        const void *hidden16, const void *X16, bool dy16_ready) {
     const int F = w[0]->dev.N;
     const size_t bf = (size_t)T * F * sizeof(float);
     if (hidden16 && !ffn_hidden16_ok(e, w, T))
@@ -767,9 +774,9 @@ int ffn_backward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *con
     if (gate_d == dh || gate_d == dg || gate_d == du || up_d == dh || up_d == dg || up_d == du ||
         (hidden_d && (hidden_d == dh || hidden_d == dg || hidden_d == du)))
         return fail(GT_ERR_INVALID, "gt_ffn_backward: gate, up and hidden must be the caller's buffers (the forward call was given NULL)");
-    const float *dy1 = dYd;
+    const float *dy1 = dy16_ready ? nullptr : dYd;
     int rc = backward_group_device(e, 1, w + 2, ad ? ad + 2 : nullptr, &dy1, hidden_d, dh, T,
-                                   (flags & ~GT_FLAG_DX_ASSIGN) | GT_FLAG_DX_ASSIGN, hidden16);      // dHidden is written, not added to
+                                   (flags & ~GT_FLAG_DX_ASSIGN) | GT_FLAG_DX_ASSIGN, hidden16, dy16_ready);      // dHidden is written, not added to
     if (rc != GT_OK) return rc;
     if (ffn_dy16_ok(e, w, T) && dXd) {
         // dGate, dUp as bf16 only, written where the group's transpose GEMM and adapter passes read their 16-bit dY

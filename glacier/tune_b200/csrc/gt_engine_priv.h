@@ -172,7 +172,10 @@ int ffn_forward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *cons
                        float *hidden_d, float *Yd, int T, int flags, void *hidden16 = nullptr, const void *X16 = nullptr);
 int ffn_backward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *const *ad, const float *dYd, const float *Xd,
                         const float *gate_d, const float *up_d, const float *hidden_d, float *dXd, int T, int flags,
-                        const void *hidden16 = nullptr, const void *X16 = nullptr);
+                        const void *hidden16 = nullptr, const void *X16 = nullptr, bool dy16_ready = false);
+// dy16_ready: the (first member's) dY is in the engine's dy16 scratch as dense bf16 [T, out], put there by its producer; the scratch
+// has been sized with this call before anything was written.
+int reserve_dy16(gt_engine *e, int n, const gt_weight *const *w, int T);
 int join_comm(gt_engine *e);
 int allreduce_begin_locked(gt_engine *e, float *g_dev, int64_t count, float scale);
 // forget the captured step of every model of this engine (before the communicator its collectives belong to goes away)

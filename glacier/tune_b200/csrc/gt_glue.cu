@@ -356,12 +356,13 @@ __global__ void __launch_bounds__(256) k_add_rmsnorm_fwd(const float *__restrict
 // dx = r * g - x * r^3 * mean(g * x), g = dy * w (frozen weight)
 // (+ residual when given: the gradient that bypasses the norm on the residual connection, TransformerBlock.cs:675,838)
 __global__ void __launch_bounds__(256) k_rmsnorm_bwd(const float *__restrict__ dy, const float *__restrict__ x, const float *__restrict__ w,
-                                                     const float *residual, float *dx, int H, float eps) {
+                                                     const float *residual, float *dx, __nv_bfloat16 *__restrict__ dx16, int H, float eps) {
     pdl_wait();
     pdl_trigger();
     const float *xr = x + (int64_t)blockIdx.x * H, *gr = dy + (int64_t)blockIdx.x * H;
     const float *rr = residual ? residual + (int64_t)blockIdx.x * H : nullptr;
     float *dr = dx + (int64_t)blockIdx.x * H;
+    __nv_bfloat16 *dr16 = dx16 ? dx16 + (int64_t)blockIdx.x * H : nullptr;      // a rounded copy as well (dx itself goes on as a residual)
     // (the residual may alias dx: its values are taken before anything is stored)
     float xv[kRowRegs], gv[kRowRegs], rv[kRowRegs];
     float ss = 0.f, gx = 0.f;
@@ -384,9 +385,17 @@ __global__ void __launch_bounds__(256) k_rmsnorm_bwd(const float *__restrict__ d
 #pragma unroll
     for (int j = 0; j < kRowRegs; j++) {
         const int i = threadIdx.x + j * 256;
-        if (i < H) dr[i] = r * gv[j] - xv[j] * coef + rv[j];
+        if (i < H) {
+            const float v = r * gv[j] - xv[j] * coef + rv[j];
+            dr[i] = v;
+            if (dr16) dr16[i] = __float2bfloat16_rn(v);
+        }
     }
-    for (int i = threadIdx.x + kRowRegs * 256; i < H; i += 256) dr[i] = r * gr[i] * w[i] - xr[i] * coef + (rr ? rr[i] : 0.f);
+    for (int i = threadIdx.x + kRowRegs * 256; i < H; i += 256) {
+        const float v = r * gr[i] * w[i] - xr[i] * coef + (rr ? rr[i] : 0.f);
+        dr[i] = v;
+        if (dr16) dr16[i] = __float2bfloat16_rn(v);
+    }
 }
 
 int aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -449,8 +458,8 @@ cudaError_t launch_rmsnorm_fwd(const float *x, const float *w, float *y, int T, 
     return launch_k(k_rmsnorm_fwd, dim3((unsigned)T), dim3(256), (size_t)0, s, x, w, y, (__nv_bfloat16 *)y16, H, eps);
 }
 cudaError_t launch_rmsnorm_bwd(const float *dy, const float *x, const float *w, const float *residual, float *dx, int T, int H, float eps,
-                               cudaStream_t s) {
-    return launch_k(k_rmsnorm_bwd, dim3((unsigned)T), dim3(256), (size_t)0, s, dy, x, w, residual, dx, H, eps);
+                               cudaStream_t s, void *dx16) {
+    return launch_k(k_rmsnorm_bwd, dim3((unsigned)T), dim3(256), (size_t)0, s, dy, x, w, residual, dx, (__nv_bfloat16 *)dx16, H, eps);
 }
 cudaError_t launch_add_rmsnorm_fwd(const float *a, const float *b, const float *w, float *sum, float *y, int T, int H, float eps, cudaStream_t s,
                                    void *y16) {

@@ -261,7 +261,7 @@ cudaError_t launch_rope(float *q, float *k, int T, int heads_q, int heads_kv, in
 cudaError_t launch_rmsnorm_fwd(const float *x, const float *w, float *y, int T, int H, float eps, cudaStream_t s, void *y16 = nullptr);
 // dx = RMSNorm backward (+ residual, which may be null and may alias dx)
 cudaError_t launch_rmsnorm_bwd(const float *dy, const float *x, const float *w, const float *residual, float *dx, int T, int H, float eps,
-                               cudaStream_t s);
+                               cudaStream_t s, void *dx16 = nullptr);
 // sum = a + b (sum may alias a or b), y = RMSNorm(sum) * w
 cudaError_t launch_add_rmsnorm_fwd(const float *a, const float *b, const float *w, float *sum, float *y, int T, int H, float eps, cudaStream_t s,
                                    void *y16 = nullptr);

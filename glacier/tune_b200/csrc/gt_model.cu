@@ -98,10 +98,12 @@ int check_ready(const gt_model *m, const char *who) {
 // attention's backward reads the fp32 output too), and neither a cast nor the adapters' products read an fp32 tensor back.
 struct Inputs16 {
     bool qkv, o, gu;
+    bool dy_o, dy_down;      // the gradients of the o and down projections' outputs come as bf16 from the norm backward before them
 };
 Inputs16 inputs16(const gt_model *m, int l, int T) {
     const LayerDev &L = m->layers[l];
-    return {group_x16_ok(m->eng, 3, L.w + kQ, T), group_x16_ok(m->eng, 1, L.w + kO, T), group_x16_ok(m->eng, 2, L.w + kGate, T)};
+    const bool h8 = m->cfg.hidden % 8 == 0, o = group_x16_ok(m->eng, 1, L.w + kO, T);
+    return {group_x16_ok(m->eng, 3, L.w + kQ, T), o, group_x16_ok(m->eng, 2, L.w + kGate, T), h8 && o, h8 && group_x16_ok(m->eng, 1, L.w + kDown, T)};
 }
 
 // One block forward on the engine stream; s receives the state.  n1_ready: s.n1 already holds RMSNorm(x_in) (the block
@@ -161,12 +163,12 @@ int block_backward(gt_model *m, int l, const float *d_out, const float *x_in, co
     const bool h16 = ffn_hidden16_ok(e, fw, T);
     const Inputs16 i16 = inputs16(m, l, T);
     int rc = ffn_backward_device(e, fw, fa, d_out, s.n2, s.gate, s.up, h16 ? nullptr : s.hidden, m->dn, T, flags,
-                                 h16 ? (const void *)s.hidden : nullptr, i16.gu ? s.n2 : nullptr);
+                                 h16 ? (const void *)s.hidden : nullptr, i16.gu ? s.n2 : nullptr, i16.dy_down);
     if (rc != GT_OK) return rc;
-    GT_LAUNCH(e, launch_rmsnorm_bwd(m->dn, s.x1, L.norm2, d_out, m->dx1, T, H, c.rms_eps, e->stream));
+    GT_LAUNCH(e, launch_rmsnorm_bwd(m->dn, s.x1, L.norm2, d_out, m->dx1, T, H, c.rms_eps, e->stream, i16.dy_o ? e->dy16.p : nullptr));
     // B. attention: o projection, attention, RoPE, q | k | v -> dNorm1X; RMSNorm1 backward + residual
-    const float *dy_o = m->dx1;
-    rc = backward_group_device(e, 1, L.w + kO, L.ad + kO, &dy_o, s.attn, m->dattn, T, flags, i16.o ? s.attn16 : nullptr);
+    const float *dy_o = i16.dy_o ? nullptr : m->dx1;
+    rc = backward_group_device(e, 1, L.w + kO, L.ad + kO, &dy_o, s.attn, m->dattn, T, flags, i16.o ? s.attn16 : nullptr, i16.dy_o);
     if (rc != GT_OK) return rc;
     rc = attention_backward16_on_device(e, m->dattn, s.q16, s.k16, s.v16, s.attn, s.lse, m->dq, m->dk, m->dv, T, c.n_heads, c.n_kv_heads, c.head_dim);
     if (rc != GT_OK) return rc;
@@ -174,7 +176,8 @@ int block_backward(gt_model *m, int l, const float *d_out, const float *x_in, co
     const float *dqkv[3] = {m->dq, m->dk, m->dv};
     rc = backward_group_device(e, 3, L.w + kQ, L.ad + kQ, dqkv, s.n1, m->dn, T, flags, i16.qkv ? s.n1 : nullptr);
     if (rc != GT_OK) return rc;
-    GT_LAUNCH(e, launch_rmsnorm_bwd(m->dn, x_in, L.norm1, m->dx1, d_in, T, H, c.rms_eps, e->stream));
+    void *const next16 = l > 0 && inputs16(m, l - 1, T).dy_down ? e->dy16.p : nullptr;      // (nothing writes dy16 until block l - 1's FFN reads it)
+    GT_LAUNCH(e, launch_rmsnorm_bwd(m->dn, x_in, L.norm1, m->dx1, d_in, T, H, c.rms_eps, e->stream, next16));
     return GT_OK;
 }
 
@@ -183,13 +186,13 @@ int stage_inputs(gt_model *m, const int32_t *tokens, const int32_t *labels, int 
     const cudaMemcpyKind kind = (flags & GT_FLAG_DEVICE_PTRS) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     GT_CUDA(cudaMemcpyAsync(m->tokens, tokens, (size_t)T * sizeof(int), kind, e->stream));
     GT_CUDA(cudaMemcpyAsync(m->labels, labels, (size_t)T * sizeof(int), kind, e->stream));
-    GT_CUDA(cudaMemsetAsync(m->bad, 0, sizeof(int), e->stream));
     return GT_OK;
 }
 
 int forward_all(gt_model *m, int T, bool keep_states) {
     gt_engine *e = m->eng;
     const int L = (int)m->layers.size();
+    GT_CUDA(cudaMemsetAsync(m->bad, 0, sizeof(int), e->stream));
     // every adapter's low and dLow of the pass, cleared in a launch or two instead of a few per block
     std::vector<gt_adapter *> lows;
     for (int l = 0; l < L; l++)
@@ -225,16 +228,18 @@ int finish_loss(gt_model *m, float *loss_out, int32_t *valid_out, int flags) {
         if (valid_out) GT_CUDA(cudaMemcpyAsync(valid_out, m->valid, sizeof(int), cudaMemcpyDeviceToDevice, e->stream));
         return GT_OK;
     }
-    float hl = 0.f;
-    int hv = 0, hb = 0;
-    GT_CUDA(cudaMemcpyAsync(&hl, m->loss, sizeof(float), cudaMemcpyDeviceToHost, e->stream));
-    GT_CUDA(cudaMemcpyAsync(&hv, m->valid, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
-    GT_CUDA(cudaMemcpyAsync(&hb, m->bad, sizeof(int), cudaMemcpyDeviceToHost, e->stream));
+    // loss, valid and bad are neighbours in the arena, 256 bytes each: one copy
+    struct {
+        float loss, pad0[63];
+        int valid, pad1[63], bad;
+    } h = {};
+    static_assert(sizeof(h) == 516, "the three scalars as they lie in the arena");
+    GT_CUDA(cudaMemcpyAsync(&h, m->loss, sizeof(h), cudaMemcpyDeviceToHost, e->stream));
     int rc = check_status(e);
     if (rc != GT_OK) return rc;
-    if (hb) return failf(GT_ERR_INVALID, "%d input token id(s) outside the vocabulary [0, %d)", hb, m->cfg.vocab);      // GgufLoraModel.cs:443-452
-    if (loss_out) *loss_out = hl;
-    if (valid_out) *valid_out = hv;
+    if (h.bad) return failf(GT_ERR_INVALID, "%d input token id(s) outside the vocabulary [0, %d)", h.bad, m->cfg.vocab);      // GgufLoraModel.cs:443-452
+    if (loss_out) *loss_out = h.loss;
+    if (valid_out) *valid_out = h.valid;
     return GT_OK;
 }
 
@@ -299,7 +304,7 @@ int gt_model_create(gt_engine *e, const gt_model_config *cfg, gt_model **out) {
     m->k = take(bk); m->v = take(bk); m->dk = take(bk); m->dv = take(bk);
     m->tokens = (int *)take(a256(T * 4));
     m->labels = (int *)take(a256(T * 4));
-    m->loss = take(256);
+    m->loss = take(256);      // loss, valid, bad: read back together
     m->valid = (int *)take(256);
     m->bad = (int *)take(256);
     m->graph_off = cfg->no_graph != 0;
@@ -459,7 +464,13 @@ int step_body(gt_model *m, int T) {
     // loss and its gradient with respect to the normed final hidden state, then through the final RMSNorm
     rc = lm_head_loss_on_device(e, m->lm_head, m->fnorm, m->labels, T, m->loss, m->valid, m->dfnorm);
     if (rc != GT_OK) return rc;
-    GT_LAUNCH(e, launch_rmsnorm_bwd(m->dfnorm, m->x[L], m->out_norm, nullptr, m->dx_a, T, H, m->cfg.rms_eps, e->stream));
+    for (int l = 0; l < L; l++) {
+        const LayerDev &D = m->layers[l];
+        for (int g = 0; g < 4 && rc == GT_OK; g++) rc = reserve_dy16(e, g == 0 ? 3 : (g == 2 ? 2 : 1), D.w + (g == 0 ? kQ : (g == 1 ? kO : (g == 2 ? kGate : kDown))), T);
+        if (rc != GT_OK) return rc;
+    }
+    GT_LAUNCH(e, launch_rmsnorm_bwd(m->dfnorm, m->x[L], m->out_norm, nullptr, m->dx_a, T, H, m->cfg.rms_eps, e->stream,
+                                    inputs16(m, L - 1, T).dy_down ? e->dy16.p : nullptr));
     float *d_cur = m->dx_a, *d_next = m->dx_b;
     const float inv_world = 1.0f / (float)e->dp_world;
     for (int l = L - 1; l >= 0; l--) {
