@@ -513,10 +513,10 @@ static size_t dy16_layout(int n, const gt_weight *const *w, int T, size_t *off, 
     return total;
 }
 
-int reserve_dy16(gt_engine *e, int n, const gt_weight *const *w, int T) {
-    size_t off[kMaxGroup];
+int reserve_dy16(gt_engine *e, int n, const gt_weight *const *w, int T, size_t *off) {
+    size_t at[kMaxGroup];
     int ld[kMaxGroup];
-    GT_CUDA(e->dy16.reserve(dy16_layout(n, w, T, off, ld)));
+    GT_CUDA(e->dy16.reserve(dy16_layout(n, w, T, off ? off : at, ld)));
     return GT_OK;
 }
 

@@ -175,7 +175,8 @@ int ffn_backward_device(gt_engine *e, const gt_weight *const *w, gt_adapter *con
                         const void *hidden16 = nullptr, const void *X16 = nullptr, bool dy16_ready = false);
 // dy16_ready: the (first member's) dY is in the engine's dy16 scratch as dense bf16 [T, out], put there by its producer; the scratch
 // has been sized with this call before anything was written.
-int reserve_dy16(gt_engine *e, int n, const gt_weight *const *w, int T);
+// off (may be null): where each member's copy goes, in bytes.
+int reserve_dy16(gt_engine *e, int n, const gt_weight *const *w, int T, size_t *off = nullptr);
 int join_comm(gt_engine *e);
 int allreduce_begin_locked(gt_engine *e, float *g_dev, int64_t count, float scale);
 // forget the captured step of every model of this engine (before the communicator its collectives belong to goes away)

@@ -220,12 +220,20 @@ __global__ void __launch_bounds__(256) k_add(const float *__restrict__ a, const 
 // One block per position: the first threads evaluate cos / sin of the position's angles once into shared memory (powf
 // and a sincosf of a large angle, repeated per head, cost more than the memory traffic), then all threads walk the
 // (head, pair) items of q and k with coalesced accesses.  freq and theta follow the reference's fp32 order.
+// q16 given (vec only): q and k go out rounded to bf16 there and in k16 instead, and v is rounded into v16 - the dY operands of the
+// q, k, v projections' backward, so that neither a cast nor the adapter pass reads fp32 gradients back.
 constexpr int kRopeMaxHalf = 256;
+struct Rope16 {
+    __nv_bfloat16 *q16, *k16, *v16;
+    const float *v;
+};
+__device__ __forceinline__ void st_bf16x4(__nv_bfloat16 *dst, float a, float b, float c, float d) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+    *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+}
 __global__ void __launch_bounds__(256) k_rope(float *__restrict__ q, float *__restrict__ k, int T, int heads_q, int heads_kv, int head_dim,
-                                              float freq_base, float freq_scale, int eff, float sign, int vec) {
+                                              float freq_base, float freq_scale, int eff, float sign, int vec, const Rope16 o) {
     __shared__ __align__(16) float cs[kRopeMaxHalf], sn[kRopeMaxHalf];
-    pdl_wait();
-    pdl_trigger();
     const int half = eff >> 1;
     const int pos = blockIdx.x;
     for (int i = threadIdx.x; i < half; i += blockDim.x) {
@@ -236,6 +244,8 @@ __global__ void __launch_bounds__(256) k_rope(float *__restrict__ q, float *__re
         cs[i] = c;
         sn[i] = s * sign;
     }
+    pdl_wait();      // (the angles need nothing of the kernel before)
+    pdl_trigger();
     __syncthreads();
     const int hq = q ? heads_q : 0, heads = hq + (k ? heads_kv : 0);
     if (vec) {      // four pairs per thread: 16-byte loads and stores of both halves
@@ -245,8 +255,23 @@ __global__ void __launch_bounds__(256) k_rope(float *__restrict__ q, float *__re
             float *p = h < hq ? q + ((int64_t)pos * heads_q + h) * head_dim + i : k + ((int64_t)pos * heads_kv + (h - hq)) * head_dim + i;
             const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + half);
             const float4 c = *reinterpret_cast<const float4 *>(cs + i), s = *reinterpret_cast<const float4 *>(sn + i);
-            *reinterpret_cast<float4 *>(p) = make_float4(a.x * c.x - b.x * s.x, a.y * c.y - b.y * s.y, a.z * c.z - b.z * s.z, a.w * c.w - b.w * s.w);
-            *reinterpret_cast<float4 *>(p + half) = make_float4(a.x * s.x + b.x * c.x, a.y * s.y + b.y * c.y, a.z * s.z + b.z * c.z, a.w * s.w + b.w * c.w);
+            const float4 u = make_float4(a.x * c.x - b.x * s.x, a.y * c.y - b.y * s.y, a.z * c.z - b.z * s.z, a.w * c.w - b.w * s.w);
+            const float4 w = make_float4(a.x * s.x + b.x * c.x, a.y * s.y + b.y * c.y, a.z * s.z + b.z * c.z, a.w * s.w + b.w * c.w);
+            if (o.q16) {
+                __nv_bfloat16 *d = h < hq ? o.q16 + (p - q) : o.k16 + (p - k);
+                st_bf16x4(d, u.x, u.y, u.z, u.w);
+                st_bf16x4(d + half, w.x, w.y, w.z, w.w);
+            } else {
+                *reinterpret_cast<float4 *>(p) = u;
+                *reinterpret_cast<float4 *>(p + half) = w;
+            }
+        }
+        if (o.q16) {
+            const int64_t v0 = (int64_t)pos * heads_kv * head_dim;
+            for (int i = threadIdx.x * 4; i < heads_kv * head_dim; i += blockDim.x * 4) {
+                const float4 a = *reinterpret_cast<const float4 *>(o.v + v0 + i);
+                st_bf16x4(o.v16 + v0 + i, a.x, a.y, a.z, a.w);
+            }
         }
         return;
     }
@@ -452,7 +477,16 @@ cudaError_t launch_rope(float *q, float *k, int T, int heads_q, int heads_kv, in
     // 16-byte accesses where every head's halves start on a 16-byte boundary
     const int vec = (eff / 2) % 4 == 0 && head_dim % 4 == 0 && (!q || aligned16(q)) && (!k || aligned16(k)) ? 1 : 0;
     return launch_k(k_rope, dim3((unsigned)T), dim3(256), (size_t)0, s, q, k, T, heads_q, heads_kv, head_dim, freq_base, freq_scale, eff,
-                    inverse ? -1.0f : 1.0f, vec);
+                    inverse ? -1.0f : 1.0f, vec, Rope16{});
+}
+// The inverse rotation of dq, dk over the whole head (head_dim % 8 == 0, up to 512) with bf16 results, and dv rounded; 16-byte
+// aligned tensors.
+cudaError_t launch_rope_bwd16(float *dq, float *dk, const float *dv, void *dq16, void *dk16, void *dv16, int T, int heads_q, int heads_kv,
+                              int head_dim, float freq_base, cudaStream_t s) {
+    if (T <= 0) return cudaSuccess;
+    if (head_dim % 8 != 0 || head_dim / 2 > kRopeMaxHalf) return cudaErrorInvalidValue;
+    return launch_k(k_rope, dim3((unsigned)T), dim3(256), (size_t)0, s, dq, dk, T, heads_q, heads_kv, head_dim, freq_base, 1.0f, head_dim, -1.0f, 1,
+                    Rope16{(__nv_bfloat16 *)dq16, (__nv_bfloat16 *)dk16, (__nv_bfloat16 *)dv16, dv});
 }
 cudaError_t launch_rmsnorm_fwd(const float *x, const float *w, float *y, int T, int H, float eps, cudaStream_t s, void *y16) {
     return launch_k(k_rmsnorm_fwd, dim3((unsigned)T), dim3(256), (size_t)0, s, x, w, y, (__nv_bfloat16 *)y16, H, eps);

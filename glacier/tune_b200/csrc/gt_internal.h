@@ -263,6 +263,8 @@ cudaError_t launch_rmsnorm_fwd(const float *x, const float *w, float *y, int T, 
 cudaError_t launch_rmsnorm_bwd(const float *dy, const float *x, const float *w, const float *residual, float *dx, int T, int H, float eps,
                                cudaStream_t s, void *dx16 = nullptr);
 // sum = a + b (sum may alias a or b), y = RMSNorm(sum) * w
+cudaError_t launch_rope_bwd16(float *dq, float *dk, const float *dv, void *dq16, void *dk16, void *dv16, int T, int heads_q, int heads_kv,
+                              int head_dim, float freq_base, cudaStream_t s);
 cudaError_t launch_add_rmsnorm_fwd(const float *a, const float *b, const float *w, float *sum, float *y, int T, int H, float eps, cudaStream_t s,
                                    void *y16 = nullptr);
 

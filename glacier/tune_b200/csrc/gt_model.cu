@@ -172,9 +172,19 @@ int block_backward(gt_model *m, int l, const float *d_out, const float *x_in, co
     if (rc != GT_OK) return rc;
     rc = attention_backward16_on_device(e, m->dattn, s.q16, s.k16, s.v16, s.attn, s.lse, m->dq, m->dk, m->dv, T, c.n_heads, c.n_kv_heads, c.head_dim);
     if (rc != GT_OK) return rc;
-    GT_LAUNCH(e, launch_rope(m->dq, m->dk, T, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_theta, 1.0f, c.head_dim, 1, e->stream));
     const float *dqkv[3] = {m->dq, m->dk, m->dv};
-    rc = backward_group_device(e, 3, L.w + kQ, L.ad + kQ, dqkv, s.n1, m->dn, T, flags, i16.qkv ? s.n1 : nullptr);
+    if (i16.qkv) {      // (heads of 128: the projections' rows are dense in the 16-bit scratch)
+        size_t off[3];
+        rc = reserve_dy16(e, 3, L.w + kQ, T, off);
+        if (rc != GT_OK) return rc;
+        char *d16 = (char *)e->dy16.p;
+        GT_LAUNCH(e, launch_rope_bwd16(m->dq, m->dk, m->dv, d16 + off[0], d16 + off[1], d16 + off[2], T, c.n_heads, c.n_kv_heads, c.head_dim,
+                                       c.rope_theta, e->stream));
+        dqkv[0] = dqkv[1] = dqkv[2] = nullptr;
+    } else {
+        GT_LAUNCH(e, launch_rope(m->dq, m->dk, T, c.n_heads, c.n_kv_heads, c.head_dim, c.rope_theta, 1.0f, c.head_dim, 1, e->stream));
+    }
+    rc = backward_group_device(e, 3, L.w + kQ, L.ad + kQ, dqkv, s.n1, m->dn, T, flags, i16.qkv ? s.n1 : nullptr, i16.qkv);
     if (rc != GT_OK) return rc;
     void *const next16 = l > 0 && inputs16(m, l - 1, T).dy_down ? e->dy16.p : nullptr;      // (nothing writes dy16 until block l - 1's FFN reads it)
     GT_LAUNCH(e, launch_rmsnorm_bwd(m->dn, x_in, L.norm1, m->dx1, d_in, T, H, c.rms_eps, e->stream, next16));
