@@ -13,12 +13,13 @@
 //   D[128 x tokens] (TMEM, fp32)  +=  Wtile[128 x 64] (SMEM, dequantized 16-bit)  x  act[tokens x 64]^T (SMEM via TMA)
 //
 // Warp roles (640 threads):
-//   warp 0        TMA producer of the packed super-blocks of W (raw bytes)
+//   warp 0        TMA producer of the packed half or whole super-blocks of W (raw bytes)
 //   warp 19       TMA producer of the 16-bit activation tiles
-//   warps 1, 18   tcgen05.mma issuers (one thread each, alternate stages, a turn token keeps the order fixed);
+//   warps 1, 18   tcgen05.mma issuers (one elected lane each, alternate stages, a turn token keeps the order fixed);
 //                 warp 1 owns the TMEM allocation
 //   warps 2-17    four groups of 4 warps that dequantize every fourth operand stage each (raw blocks -> 128-byte-
-//                 swizzled tiles); afterwards all 16 run the epilogue (tcgen05.ld -> bias -> global store / atomic add)
+//                 swizzled tiles); all 16 build the rank-update stages and run the epilogue (tcgen05.ld -> bias -> global
+//                 store / atomic add)
 //
 // One launch serves up to three member projections (forward: they share the activation tiles, each tile index belongs
 // to one member; backward: their contraction ranges are concatenated and all sum into one dX), each with its own
